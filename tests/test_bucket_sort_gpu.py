@@ -1,0 +1,86 @@
+"""Whole-key sorts of 4- and 8-byte keys that may take the bucket plan (one or two radix passes on the top bits, then
+the buckets in shared memory) against the CPU oracle — bit exact, whichever way the device decides.
+
+The inputs reach every decision: buckets that fit after one pass and after two, tiles of whole groups and cut tiles,
+keys outside the sampled window, a bucket above the capacity, 64-bit keys whose windows are equal, crowded bins.
+"""
+import ctypes as C
+
+import numpy as np
+import pytest
+import torch
+
+import oracle
+import thrust_b200 as tb
+from thrust_b200 import _capi as capi
+from util import random_keys, to_device, to_host
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [9217, 16385, 100003, 1180003, 4200001]  # one pass, its end for evenly spread keys, two passes
+
+
+def _keys(rng, kind, n, dtype):
+    dt = np.dtype(dtype)
+    u = np.dtype(f"u{dt.itemsize}")
+    bits = 8 * dt.itemsize
+    raw = random_keys(rng, n, u)
+    if kind == "window":  # a common prefix above 26 bits (32-bit keys) or 50 bits
+        raw = (raw >> u.type(bits - (26 if bits == 32 else 50))) | u.type(1 << (bits - 2))
+    elif kind == "outlier":  # too few for the sample to see
+        raw >>= u.type(4)
+        raw[n // 3] = np.iinfo(u).max
+        raw[n // 2] = 0
+    elif kind == "heavy":  # one value 12000 times: no bucket of its own
+        raw[rng.choice(n, size=min(n // 2, 12000), replace=False)] = raw[0]
+    elif kind == "low":  # few distinct prefixes of 40 bits: equal windows, crowded bins
+        raw = (raw >> u.type(bits - 20)) << u.type(bits - 20) | random_keys(rng, n, u, bits=6)
+    elif kind == "normal":
+        f = np.float32 if bits == 32 else np.float64
+        raw = rng.standard_normal(n).astype(f).view(u)
+    return raw.view(dtype)
+
+
+@pytest.mark.parametrize("kind", ["uniform", "window", "outlier", "heavy", "low", "normal"])
+@pytest.mark.parametrize("dtype", [np.int32, np.float32, np.uint64, np.float64])
+def test_bucket_plan(cuda_device, dtype, kind):
+    chk = oracle.port()
+    for n in SIZES:
+        rng = np.random.default_rng(8000 + n)
+        k = _keys(rng, kind, n, dtype)
+        desc = n == 100003
+        v = np.arange(n, dtype=np.uint32)
+        dk, dv = to_device(k, offset_elems=n % 3), to_device(v)
+        tb.sort_by_key(dk, dv, descending=desc)
+        wk, wv = chk.sort_by_key(k, v, desc)
+        assert to_host(dk, dtype).tobytes() == wk.tobytes(), n
+        assert to_host(dv, np.uint32).tobytes() == wv.tobytes(), (n, "values (stability)")
+        d = to_device(k)
+        tb.sort(d, descending=desc)
+        assert to_host(d, dtype).tobytes() == wk.tobytes(), (n, "keys only")
+
+
+@pytest.mark.parametrize("vbytes", [1, 2, 8, 16])
+@pytest.mark.parametrize("dtype", [np.uint32, np.int64])
+def test_bucket_plan_value_widths(cuda_device, dtype, vbytes):
+    n = 1500007
+    rng = np.random.default_rng(8100)
+    k = random_keys(rng, n, dtype)
+    v = rng.integers(0, 256, size=(n, vbytes), dtype=np.uint8)
+    order = np.argsort(k, kind="stable")
+    dk, dv = to_device(k), to_device(v.reshape(-1))
+    need = C.c_size_t(0)
+    kd = tb.tb200_dtype(dk)
+    stream = C.c_void_p(torch.cuda.current_stream(cuda_device).cuda_stream)
+    args = (n, kd, vbytes, 0, 0, 8 * k.itemsize, stream)
+    capi.check(capi.lib.tb200_radix_sort(None, C.byref(need), None, None, *args), "size")
+    temp = torch.empty(need.value, dtype=torch.uint8, device=cuda_device)
+    # once with all of the scratch, once with what the byte-wise passes alone need
+    for cut in (0, 1 << 19):
+        have = C.c_size_t(need.value - cut)
+        a, b = dk.clone(), dv.clone()
+        capi.check(capi.lib.tb200_radix_sort(C.c_void_p(temp.data_ptr()), C.byref(have), C.c_void_p(a.data_ptr()),
+                                             C.c_void_p(b.data_ptr()), *args), "sort")
+        capi.check(capi.lib.tb200_temp_status(C.c_void_p(temp.data_ptr()), stream), "status")
+        assert to_host(a, dtype).tobytes() == k[order].tobytes(), cut
+        assert to_host(b, np.uint8).tobytes() == v[order].tobytes(), cut

@@ -26,6 +26,7 @@
 // rest (bitwise total order); descending -> complement.
 #include "sort_common.cuh"
 #include "block_sort.cuh"
+#include "bucket_sort.cuh"
 
 namespace tb200 {
 namespace {
@@ -161,6 +162,7 @@ histogram_bytes_kernel(const UK* __restrict__ keys, uint64_t n, Encoding enc, So
   extern __shared__ __align__(16) unsigned s_cnt[];  // [P][128][32]
   __shared__ unsigned s_last;
   __shared__ unsigned long long s_warp_tot[8];
+  if (ctl->bucket_mode) return;  // the bucket plan brings the offsets of its own digits
 
   const unsigned lane = lane_id();
   for (int i = threadIdx.x; i < kEntries * kWarp; i += T) s_cnt[i] = 0;
@@ -420,8 +422,12 @@ onesweep_kernel(const PassParams prm) {
   const unsigned warp = threadIdx.x / kWarp;
   const unsigned lane = lane_id();
   const unsigned warp_off = warp * Shape::kWarpItems;
-  const int shift = prm.shift;
-  const unsigned mask = prm.mask;
+  int shift = prm.shift;
+  unsigned mask = prm.mask;
+  if (!SPLIT && ctl->bucket_mode) {  // passes 0 and 1 of a bucket plan (later ones are skipped)
+    shift = (int)ctl->pass_shift[pass];
+    mask = ctl->pass_mask[pass];
+  }
   const unsigned num_tiles = prm.num_tiles;
   unsigned* whist = s_whist + warp * kRadix;
   const unsigned num_split = SPLIT ? prm.num_splitters : 0u;
@@ -836,8 +842,9 @@ int sort_impl(void* d_temp, size_t* temp_bytes, void* d_keys, void* d_vals, uint
   const uint64_t tiles = (n + TILE - 1) / TILE;
   const bool wide = n > (1ull << 30);
   const Layout lay = make_layout(n, sizeof(UK), VB, tiles, wide ? 8 : 4);
+  const size_t bucket_bytes = bucket_scratch_bytes(n, sizeof(UK), VB);
   if (d_temp == nullptr) {
-    *temp_bytes = lay.total;
+    *temp_bytes = lay.total + bucket_bytes;
     return TB200_OK;
   }
   if (*temp_bytes < lay.total) return TB200_ERR_TEMP_TOO_SMALL;
@@ -857,7 +864,15 @@ int sort_impl(void* d_temp, size_t* temp_bytes, void* d_keys, void* d_vals, uint
     if (d_keys == nullptr || (VB && d_vals == nullptr)) return TB200_ERR_INVALID_ARGUMENT;
     return block_sort_single(d_keys, d_vals, n, sizeof(UK), VB, kind, descending, &ctl->status, stream);
   }
-  if (phase != kPhaseFinish) TB200_CUDA_TRY(cudaMemsetAsync(d_temp, 0, lay.clear_bytes, stream));
+  // Larger whole-key sorts try a bucket plan first (a scratch sized for the byte-wise sort alone still serves that).
+  const bool buckets = phase == kPhaseAll && whole && bucket_bytes != 0 && *temp_bytes >= lay.total + bucket_bytes;
+  if (buckets) {
+    if (d_keys == nullptr || (VB && d_vals == nullptr)) return TB200_ERR_INVALID_ARGUMENT;
+    const int rc = bucket_plan(ctl, lay.clear_bytes, base + lay.total, d_keys, n, sizeof(UK), VB, kind, descending, stream);
+    if (rc) return rc;
+  } else if (phase != kPhaseFinish) {
+    TB200_CUDA_TRY(cudaMemsetAsync(d_temp, 0, lay.clear_bytes, stream));
+  }
   if (phase == kPhaseBegin) return TB200_OK;
   if (d_keys == nullptr || (VB && d_vals == nullptr)) return TB200_ERR_INVALID_ARGUMENT;
 
@@ -935,6 +950,9 @@ int sort_impl(void* d_temp, size_t* temp_bytes, void* d_keys, void* d_vals, uint
                          PassTag<UK, VB, unsigned, false>{});
   if (rc) return rc;
 
+  if (buckets)
+    return bucket_finish(ctl, base + lay.total, d_keys, prm.keys_alt, d_vals, prm.vals_alt, n, sizeof(UK), VB, kind,
+                         descending, stream);
   copy_back_kernel<<<sms * 4, 256, 0, stream>>>(
       static_cast<uint4*>(d_keys), reinterpret_cast<const uint4*>(base + lay.keys_off), n * sizeof(UK),
       static_cast<uint4*>(d_vals), reinterpret_cast<const uint4*>(base + lay.vals_off), n * (uint64_t)VB, ctl);

@@ -20,6 +20,17 @@ struct SortCtl {
   unsigned tickets[kMaxPasses];  // dynamic tile counters, one per pass
   unsigned skip[kMaxPasses];
   unsigned exec_before[kMaxPasses];  // executed passes before pass p (ping-pong parity)
+  // Bucket plan (bucket_sort.cu). bucket_mode != 0: passes 0 and 1 take the digits below instead of bytes 0 and 1,
+  // every later pass is skipped, and the tiles listed behind the plan are sorted in shared memory.
+  unsigned bucket_mode;
+  unsigned pass_shift[2], pass_mask[2];
+  unsigned window_ok;            // the sample found a window that looks worth counting
+  unsigned window_bits;          // keys differ below this bit only
+  unsigned bucket_bits;          // the buckets are told apart by the top bucket_bits of the window
+  unsigned joint_done;           // CTAs of the bucket count that have finished
+  unsigned num_bucket_tiles;
+  unsigned tile_bits;            // the keys of one tile differ below this bit only
+  unsigned long long window_prefix;  // what all keys hold above the window
   unsigned long long hist[kMaxPasses][kRadix];
   unsigned long long offs[kMaxPasses][kRadix];
 };
