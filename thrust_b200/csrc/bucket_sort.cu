@@ -44,6 +44,7 @@ template <typename UK>
 __global__ void __launch_bounds__(kCountThreads)
 bucket_prepare_kernel(const UK* __restrict__ keys, uint64_t n, Encoding enc, SortCtl* ctl, uint64_t clear_bytes,
                       BucketScratch* scratch, int min_bits, int max_bits, unsigned capacity, int aligned) {
+  chain_begin();
   constexpr uint64_t kCtlBytes = align_up(sizeof(SortCtl), 256);
   char* base = reinterpret_cast<char*>(ctl);
   const uint4 zero = make_uint4(0, 0, 0, 0);
@@ -317,6 +318,7 @@ bucket_count_kernel(const UK* __restrict__ keys, uint64_t n, Encoding enc, SortC
   constexpr int UNROLL = 4;
   extern __shared__ __align__(16) unsigned s_mem[];  // 2^(bucket_bits - 1) words, two counters each
   __shared__ unsigned s_last;
+  chain_begin();
   if (!ctl->window_ok) return;
   const unsigned window_bits = ctl->window_bits;
   const int bucket_bits = (int)ctl->bucket_bits;
@@ -370,6 +372,7 @@ bucket_sort_kernel(UK* main_keys, UK* alt_keys, typename ValueOf<VB>::type* main
   using B = BlockSort<UK, VB, THREADS, ITEMS, BINS>;
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ unsigned s_red[B::kRedWords];
+  chain_begin();
   const bool odd = ctl->total_exec & 1u;
   if (!ctl->bucket_mode) {
     if (odd) {
@@ -433,20 +436,21 @@ int plan(SortCtl* ctl, size_t clear_bytes, BucketScratch* scratch, const UK* key
   const uint64_t vecs = (clear_bytes + (sizeof(unsigned) << max_bits)) / 16;
   const int aligned = reinterpret_cast<uintptr_t>(keys) % 16 == 0;
   const uint64_t want = 2 + vecs / (4 * kCountThreads);
-  bucket_prepare_kernel<UK><<<(unsigned)(want < (uint64_t)sms ? want : (uint64_t)sms), kCountThreads, 0, stream>>>(
-      keys, n, enc, ctl, clear_bytes, scratch, min_bits, max_bits, (unsigned)capacity, aligned);
+  TB200_CUDA_TRY(launch_chained(bucket_prepare_kernel<UK>, (unsigned)(want < (uint64_t)sms ? want : (uint64_t)sms),
+                                kCountThreads, 0, stream, keys, n, enc, ctl, (uint64_t)clear_bytes, scratch, min_bits,
+                                max_bits, (unsigned)capacity, aligned));
   trace_mark(stream, kTraceSortPlan);
-  TB200_CUDA_TRY(cudaGetLastError());
   auto kernel = bucket_count_kernel<UK>;
   constexpr size_t kMaxSmem = sizeof(uint16_t) << kMaxBucketBits;
   int per_sm = 0;
   rc = resident_ctas<CountTag<UK>>(kernel, kCountThreads, kMaxSmem, &per_sm);
   if (rc) return rc;
   const uint64_t ctas = (n + 32767) / 32768;
-  kernel<<<(unsigned)(ctas < (uint64_t)sms ? ctas : (uint64_t)sms), kCountThreads, sizeof(uint16_t) << max_bits, stream>>>(
-      keys, n, enc, ctl, scratch, (unsigned)capacity, aligned);
+  TB200_CUDA_TRY(launch_chained(kernel, (unsigned)(ctas < (uint64_t)sms ? ctas : (uint64_t)sms), kCountThreads,
+                                sizeof(uint16_t) << max_bits, stream, keys, n, enc, ctl, scratch, (unsigned)capacity,
+                                aligned));
   trace_mark(stream, kTraceSortPlan);
-  return (int)cudaGetLastError();
+  return TB200_OK;
 }
 
 template <typename UK, int VB, int SIZE>
@@ -461,11 +465,11 @@ int finish(const SortCtl* ctl, const BucketScratch* scratch, void* keys, void* k
   if (rc) return rc;
   rc = resident_ctas<TileTag<UK, VB, SIZE>>(kernel, S::kThreads, B::kSmem, &per_sm);
   if (rc) return rc;
-  kernel<<<(unsigned)(per_sm * sms), S::kThreads, B::kSmem, stream>>>(
-      static_cast<UK*>(keys), static_cast<UK*>(keys_alt), static_cast<typename B::V*>(vals),
-      static_cast<typename B::V*>(vals_alt), n, enc, ctl, scratch);
+  TB200_CUDA_TRY(launch_chained(kernel, (unsigned)(per_sm * sms), S::kThreads, B::kSmem, stream, static_cast<UK*>(keys),
+                                static_cast<UK*>(keys_alt), static_cast<typename B::V*>(vals),
+                                static_cast<typename B::V*>(vals_alt), n, enc, ctl, scratch));
   trace_mark(stream, kTraceSortTiles);
-  return (int)cudaGetLastError();
+  return TB200_OK;
 }
 
 template <typename UK, int VB>

@@ -210,6 +210,30 @@ __device__ __forceinline__ bool mbar_wait_bounded(unsigned long long* bar, unsig
   return false;
 }
 
+// Chained launches: a kernel launched with launch_chained may be brought onto the SMs while the kernel in front of it
+// in the stream still drains, which hides its launch latency. It waits in chain_begin(), which must be its first
+// statement on every path, until the kernel in front has completed and its writes are visible; from there on the
+// next kernel of the chain may be brought in.
+__device__ __forceinline__ void chain_begin() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <typename... P, typename... A>
+inline cudaError_t launch_chained(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream,
+                                  A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 #endif  // __CUDACC__
 
 }  // namespace tb200

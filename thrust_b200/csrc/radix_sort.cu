@@ -82,6 +82,7 @@ histogram_kernel(const UK* __restrict__ keys, uint64_t n, int begin_bit, int end
   __shared__ unsigned s_hist[P][kRadix];
   __shared__ unsigned s_last;
   __shared__ unsigned long long s_warp_tot[8];
+  chain_begin();
 
   for (int i = threadIdx.x; i < P * kRadix; i += kHistThreads) (&s_hist[0][0])[i] = 0;
   __syncthreads();
@@ -162,6 +163,7 @@ histogram_bytes_kernel(const UK* __restrict__ keys, uint64_t n, Encoding enc, So
   extern __shared__ __align__(16) unsigned s_cnt[];  // [P][128][32]
   __shared__ unsigned s_last;
   __shared__ unsigned long long s_warp_tot[8];
+  chain_begin();
   if (ctl->bucket_mode) return;  // the bucket plan brings the offsets of its own digits
 
   const unsigned lane = lane_id();
@@ -403,6 +405,7 @@ onesweep_kernel(const PassParams prm) {
 
   SortCtl* ctl = prm.ctl;
   const int pass = prm.pass;
+  chain_begin();
   if (ctl->skip[pass]) return;
   const unsigned before = ctl->exec_before[pass];
   const bool first_exec = before == 0;
@@ -790,6 +793,7 @@ __global__ void __launch_bounds__(256)
 copy_back_kernel(uint4* __restrict__ keys_main, const uint4* __restrict__ keys_alt, uint64_t key_bytes,
                  uint4* __restrict__ vals_main, const uint4* __restrict__ vals_alt, uint64_t val_bytes,
                  const SortCtl* ctl) {
+  chain_begin();
   if ((ctl->total_exec & 1u) == 0) return;
   copy_back(keys_main, keys_alt, key_bytes);
   if (val_bytes) copy_back(vals_main, vals_alt, val_bytes);
@@ -901,13 +905,14 @@ int sort_impl(void* d_temp, size_t* temp_bytes, void* d_keys, void* d_vals, uint
       if (prc) return prc;
       const uint64_t resident = (uint64_t)per_sm * sms;
       const unsigned grid = (unsigned)(want < resident ? (want ? want : 1) : resident);
-      kernel<<<grid, kByteHistThreads, kSmem, stream>>>(static_cast<const UK*>(d_keys), n, enc, ctl, aligned);
+      TB200_CUDA_TRY(launch_chained(kernel, grid, kByteHistThreads, kSmem, stream, static_cast<const UK*>(d_keys), n, enc,
+                                    ctl, aligned));
     } else {
       const uint64_t chunk = (uint64_t)kHistThreads * (16 / sizeof(UK)) * kHistUnroll;
       const uint64_t want = (n + chunk - 1) / chunk;
       const unsigned grid = (unsigned)(want < (uint64_t)sms * 4 ? want : (uint64_t)sms * 4);
-      histogram_kernel<UK><<<grid, kHistThreads, 0, stream>>>(static_cast<const UK*>(d_keys), n, begin_bit,
-                                                              end_bit, num_passes, enc, ctl, aligned);
+      TB200_CUDA_TRY(launch_chained(histogram_kernel<UK>, grid, kHistThreads, 0, stream, static_cast<const UK*>(d_keys), n,
+                                    begin_bit, end_bit, num_passes, enc, ctl, aligned));
     }
     trace_mark(stream, kTraceSortHistogram);
     TB200_CUDA_TRY(cudaGetLastError());
@@ -938,9 +943,8 @@ int sort_impl(void* d_temp, size_t* temp_bytes, void* d_keys, void* d_vals, uint
       prm.shift = begin_bit + 8 * p;
       const int bits = end_bit - prm.shift < 8 ? end_bit - prm.shift : 8;
       prm.mask = (1u << bits) - 1u;
-      kernel<<<grid, T::kThreads, Shape::kSmem, stream>>>(prm);
+      TB200_CUDA_TRY(launch_chained(kernel, grid, T::kThreads, Shape::kSmem, stream, prm));
       trace_mark(stream, kTraceSortPass);
-      TB200_CUDA_TRY(cudaGetLastError());
     }
     return TB200_OK;
   };
@@ -953,11 +957,12 @@ int sort_impl(void* d_temp, size_t* temp_bytes, void* d_keys, void* d_vals, uint
   if (buckets)
     return bucket_finish(ctl, base + lay.total, d_keys, prm.keys_alt, d_vals, prm.vals_alt, n, sizeof(UK), VB, kind,
                          descending, stream);
-  copy_back_kernel<<<sms * 4, 256, 0, stream>>>(
-      static_cast<uint4*>(d_keys), reinterpret_cast<const uint4*>(base + lay.keys_off), n * sizeof(UK),
-      static_cast<uint4*>(d_vals), reinterpret_cast<const uint4*>(base + lay.vals_off), n * (uint64_t)VB, ctl);
+  TB200_CUDA_TRY(launch_chained(
+      copy_back_kernel, sms * 4, 256, 0, stream, static_cast<uint4*>(d_keys),
+      reinterpret_cast<const uint4*>(base + lay.keys_off), n * sizeof(UK), static_cast<uint4*>(d_vals),
+      reinterpret_cast<const uint4*>(base + lay.vals_off), n * (uint64_t)VB, ctl));
   trace_mark(stream, kTraceSortCopyBack);
-  return (int)cudaGetLastError();
+  return TB200_OK;
 }
 
 // ---------------------------------------------------------------------------------
