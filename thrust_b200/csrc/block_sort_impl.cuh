@@ -2,16 +2,17 @@
 //
 // A radix pass over the whole array costs a launch, a look-back chain and eight ballots per key whatever the
 // size; a range that fits one CTA needs none of that. The CTA
-//   1. holds its keys in registers and finds the smallest and the largest 32-bit window of the bits that vary,
-//   2. counts them in a few thousand bins that divide [min, max] evenly: one shared-memory atomic per key, whose
+//   1. parks its keys (and values) in shared memory as they come and finds the smallest and the largest 32-bit
+//      window of the bits that vary,
+//   2. counts the keys in a few thousand bins that divide [min, max] evenly: one shared-memory atomic per key, whose
 //      return value is the key's (arbitrary) rank inside its bin. Counters are 8 bits wide, four to a word: an
 //      overflow changes the sum of all counters, and then the other way below is taken,
-//   3. scans the words of four bins and drops every key (and, in bins of two and more, its original position) at
-//      its place,
-//   4. repairs the order inside each bin: a key's place is the number of (key, position) pairs of its bin below
-//      its own, so equal keys come out in input order whatever order the atomics took. Bins hold half a key on
-//      average; a warp needs about three compares per key,
-//   5. drops keys and values at their final places and writes them out with consecutive lanes.
+//   3. scans the words of four bins and drops every key's 16-bit index at its place,
+//   4. repairs the order inside the bins of two and more by (key, index), so equal keys come out in input order
+//      whatever order the atomics took. Bins hold a quarter of a key on average: one key in nine is the second of
+//      its bin, and the warp that placed it sorts the bin; each warp gathers its bins in a list first, so that its
+//      lanes work side by side,
+//   5. gathers keys and values through the indices and writes them out with consecutive lanes.
 // Keys that crowd into few bins (kCrowd or more in one) take the other way: a least-significant-digit radix sort in
 // shared memory over the bits in which the keys differ, ranked by warp match; no input is slow beyond that, and
 // none is refused.
@@ -37,15 +38,21 @@ struct BlockSort {
   static constexpr int kWords = kRealWords + kPadBins / 4;
   static constexpr int kWordsPerThread = ((kWords + THREADS - 1) / THREADS) | 1;
   static constexpr int kBinBits = 31 - __builtin_clz((unsigned)BINS);
-  static constexpr size_t kKeysBytes = align_up((size_t)kCap * (sizeof(UK) > 4 ? sizeof(UK) : 4), 16);  // or windows
-  // counters and the scan of their words (or the digit counters of the radix way), then the positions; the values
-  // overlay all of it
+  // Shared memory: keys, values (beside the keys, or in their place once the keys are out), counters and the scan of
+  // their words (later the warps' lists; or the digit counters of the radix way), indices.
   static constexpr size_t kBinBytes = (size_t)kWords * sizeof(uint2);
   static constexpr size_t kRadixBytes = (size_t)kWarps * kRadix * sizeof(unsigned);
   static constexpr size_t kCountBytes = kBinBytes > kRadixBytes ? kBinBytes : kRadixBytes;
-  static constexpr size_t kWorkBytes = kCountBytes + align_up((size_t)kCap * 2, 16);
-  static constexpr size_t kValsBytes = align_up((size_t)kCap * VB, 16);
-  static constexpr size_t kSmem = kKeysBytes + (kWorkBytes > kValsBytes ? kWorkBytes : kValsBytes);
+  static constexpr size_t kIndexBytes = align_up((size_t)kCap * 2, 16);
+  static constexpr size_t kParkBytes = align_up((size_t)kCap * sizeof(UK), 16) + align_up((size_t)kCap * VB, 16);
+  static constexpr size_t kTurnBytes = align_up((size_t)kCap * (sizeof(UK) > VB ? sizeof(UK) : VB), 16);
+  static constexpr size_t kSmemOfCta = (size_t)227 * 1024 / (THREADS <= 512 ? 2 : 1) - 2048;
+  static constexpr bool kBeside = VB != 0 && kParkBytes + kCountBytes + kIndexBytes <= kSmemOfCta;
+  static constexpr size_t kCountOff = kBeside ? kParkBytes : kTurnBytes;
+  static constexpr size_t kIndexOff = kCountOff + kCountBytes;
+  static constexpr size_t kSmem = kIndexOff + kIndexBytes;
+  static constexpr int kListEntries = (int)(kCountBytes / 4 / kWarps);  // per warp
+  static_assert(kListEntries >= 2 * kWarp, "a list is emptied when the next keys might not fit");
   static constexpr int kRedWords = 3 * kWarps;  // static shared words the caller provides
   static_assert(kCap < 65536, "places are 16-bit");
   static_assert(kCap / kPadBins < 256 && THREADS % kPadBins == 0, "the padding's counters are 8 bits wide too");
@@ -88,9 +95,8 @@ struct BlockSort {
   __device__ __noinline__ static void radix_way(const UK* src_keys, const V* src_vals, UK* dst_keys, V* dst_vals,
                                                 unsigned m, const Encoding enc, unsigned char* smem, unsigned* s_red) {
     UK* s_keys = reinterpret_cast<UK*>(smem);
-    unsigned* s_count = reinterpret_cast<unsigned*>(smem + kKeysBytes);
-    unsigned short* s_pos = reinterpret_cast<unsigned short*>(smem + kKeysBytes + kCountBytes);
-    V* s_vals = reinterpret_cast<V*>(smem + kKeysBytes);
+    unsigned* s_count = reinterpret_cast<unsigned*>(smem + kCountOff);
+    unsigned short* s_pos = reinterpret_cast<unsigned short*>(smem + kIndexOff);
     const unsigned lane = lane_id(), warp = threadIdx.x / kWarp;
     const unsigned first = warp * (kWarp * ITEMS) + lane;
     const unsigned lt_mask = lanemask_lt();
@@ -157,7 +163,7 @@ struct BlockSort {
         if constexpr (VB != 0) at[j] = s_pos[first + j * kWarp];
       }
     }
-    // the values are fetched in sorted order while the source is still whole, then both are laid out
+    // the values are fetched in sorted order while the source is still whole
     V val[VB ? ITEMS : 1];
     if constexpr (VB != 0) {
 #pragma unroll
@@ -168,88 +174,54 @@ struct BlockSort {
 #pragma unroll
     for (int j = 0; j < ITEMS; ++j) {
       if (first + j * kWarp < m) {
-        s_keys[first + j * kWarp] = key[j];
-        if constexpr (VB != 0) s_vals[first + j * kWarp] = val[j];
+        dst_keys[first + j * kWarp] = decode_key(key[j], enc);
+        if constexpr (VB != 0) dst_vals[first + j * kWarp] = val[j];
       }
     }
-    __syncthreads();
-    write_out(dst_keys, dst_vals, s_keys, s_vals, m, enc);
-  }
-
-  __device__ static void write_out(UK* dst_keys, V* dst_vals, const UK* s_keys, const V* s_vals, unsigned m,
-                                   const Encoding& enc) {
-    UK* to_keys = dst_keys + threadIdx.x;
-    V* to_vals = VB ? dst_vals + threadIdx.x : nullptr;
-    const UK* from_keys = s_keys + threadIdx.x;
-    const V* from_vals = s_vals + threadIdx.x;
-    const int have = ((int)m - (int)threadIdx.x + THREADS - 1) / THREADS;
-    auto write = [&](auto plain) {
-      UK key[ITEMS];
-#pragma unroll
-      for (int j = 0; j < ITEMS; ++j) key[j] = from_keys[j * THREADS];
-#pragma unroll
-      for (int j = 0; j < ITEMS; ++j)
-        if (j < have) to_keys[j * THREADS] = decltype(plain)::value ? key[j] : decode_key(key[j], enc);
-      if constexpr (VB != 0) {
-        V val[ITEMS];
-#pragma unroll
-        for (int j = 0; j < ITEMS; ++j) val[j] = from_vals[j * THREADS];
-#pragma unroll
-        for (int j = 0; j < ITEMS; ++j)
-          if (j < have) to_vals[j * THREADS] = val[j];
-      }
-    };
-    if ((enc.cmask | enc.dmask) == 0) write(std::true_type{});
-    else write(std::false_type{});
   }
 
   // Sorts m <= kCap elements (m >= 1) from src to dst, which may be the same arrays. ENCODE: the source holds raw
   // keys. The keys are decoded on their way out. All keys agree above bit shift + 32 (shift < 0: find out here); the
-  // fewer bits vary below that, the better the windows tell the keys apart.
+  // fewer bits vary below that, the better the bins tell the keys apart.
   template <bool ENCODE>
   __device__ static void sort(const UK* src_keys, const V* src_vals, UK* dst_keys, V* dst_vals, unsigned m, int shift,
                               const Encoding& enc, unsigned char* smem, unsigned* s_red) {
     UK* s_keys = reinterpret_cast<UK*>(smem);
-    unsigned* s_win = reinterpret_cast<unsigned*>(smem);  // the windows, until the keys are dropped at their places
-    uint2* s_bins = reinterpret_cast<uint2*>(smem + kKeysBytes);  // x: four counters, y: elements in front of them
-    unsigned short* s_pos = reinterpret_cast<unsigned short*>(smem + kKeysBytes + kCountBytes);
-    V* s_vals = reinterpret_cast<V*>(smem + kKeysBytes);
+    V* s_vals = reinterpret_cast<V*>(smem + (kBeside ? align_up((size_t)kCap * sizeof(UK), 16) : 0));
+    uint2* s_bins = reinterpret_cast<uint2*>(smem + kCountOff);  // x: four counters, y: elements in front of them
+    unsigned short* s_index = reinterpret_cast<unsigned short*>(smem + kIndexOff);
     const unsigned lane = lane_id(), warp = threadIdx.x / kWarp;
     const unsigned first = warp * (kWarp * ITEMS) + lane;  // element j of this thread: first + 32 j
+
     // Elements behind the last one are copies of it that count in bins of their own and come out behind all others,
     // so that no step but the last store depends on m (branches around single elements cost more registers than
     // there are). `have`: elements j < have of this thread exist.
     const int have = ((int)m - (int)first + kWarp - 1) / kWarp;
     const bool all = (warp + 1) * (kWarp * ITEMS) <= m;
-    auto load = [&](const auto* src, auto& out, auto anew) {
-      auto one = [&](unsigned i) {  // `anew`: a load that the compiler cannot take for an earlier one
-        if constexpr (decltype(anew)::value) return __ldcg(src + i);
-        else return src[i];
-      };
+    auto load = [&](const auto* src, auto& out) {
       if (all) {
         src += first;  // constant offsets from one address
 #pragma unroll
-        for (int j = 0; j < ITEMS; ++j) out[j] = one(j * kWarp);
+        for (int j = 0; j < ITEMS; ++j) out[j] = src[j * kWarp];
       } else {
 #pragma unroll
-        for (int j = 0; j < ITEMS; ++j) out[j] = one(min(first + j * kWarp, m - 1));
-      }
-    };
-    // A thread keeps the windows of its keys. 64-bit keys are read a second time (from L2) when their places are
-    // known: held in registers all along they would halve the number of warps.
-    auto load_keys = [&](UK (&key)[ITEMS], auto anew) {
-      load(src_keys, key, anew);
-      if constexpr (ENCODE) {
-#pragma unroll
-        for (int j = 0; j < ITEMS; ++j) key[j] = encode_key(key[j], enc);
+        for (int j = 0; j < ITEMS; ++j) out[j] = src[min(first + j * kWarp, m - 1)];
       }
     };
     static_assert(sizeof(uint2) * kWords % 16 == 0, "cleared 16 bytes at a time");
     unsigned win[ITEMS];
     {
       UK key[ITEMS];
-      load_keys(key, std::false_type{});
+      load(src_keys, key);
+      V val[kBeside ? ITEMS : 1];
+      if constexpr (kBeside) load(src_vals, val);
       for (int w = threadIdx.x; w < kWords / 2; w += THREADS) reinterpret_cast<uint4*>(s_bins)[w] = make_uint4(0, 0, 0, 0);
+      if constexpr (ENCODE) {
+#pragma unroll
+        for (int j = 0; j < ITEMS; ++j) key[j] = encode_key(key[j], enc);
+      }
+#pragma unroll
+      for (int j = 0; j < ITEMS; ++j) s_keys[first + j * kWarp] = key[j];
       if (sizeof(UK) == 8 && shift < 0) {
         const UK ref = load_key<ENCODE>(src_keys, 0, m, enc);
         unsigned hi = 0;
@@ -263,6 +235,10 @@ struct BlockSort {
       }
 #pragma unroll
       for (int j = 0; j < ITEMS; ++j) win[j] = window(key[j], shift);
+      if constexpr (kBeside) {
+#pragma unroll
+        for (int j = 0; j < ITEMS; ++j) s_vals[first + j * kWarp] = val[j];
+      }
     }
     unsigned mn = ~0u, mx = 0;
 #pragma unroll
@@ -283,7 +259,7 @@ struct BlockSort {
     const unsigned bin0 = mn >> narrow;
     const unsigned pad_bin = BINS + threadIdx.x % kPadBins;
 
-    unsigned at[ITEMS];  // bin | rank inside the bin << 16, later place of the bin | size << 16 | rank << 22 | below << 27
+    unsigned at[ITEMS];  // bin | rank inside the bin << 16
 #pragma unroll
     for (int j = 0; j < ITEMS; ++j) {
       unsigned bin = (win[j] >> narrow) - bin0;
@@ -305,21 +281,30 @@ struct BlockSort {
       sum = __dp4a(cnt[i], 0x01010101u, sum);
       if (w0 + i < (unsigned)kRealWords) full |= cnt[i];
     }
-    unsigned run = scan_threads(sum, s_red + 2 * kWarps);
-    if (__syncthreads_or((full & kCrowdMask) != 0 || (threadIdx.x == THREADS - 1 && run + sum != (unsigned)kCap))) {
+    unsigned incl = sum;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const unsigned t = __shfl_up_sync(0xffffffffu, incl, off);
+      if (lane >= (unsigned)off) incl += t;
+    }
+    const unsigned crowd = __any_sync(0xffffffffu, (full & kCrowdMask) != 0) ? 1u << 31 : 0u;
+    if (lane == 31) s_red[2 * kWarps + warp] = incl | crowd;
+    __syncthreads();
+    const unsigned of_warp = lane < (unsigned)kWarps ? s_red[2 * kWarps + lane] : 0u;
+    const unsigned total = __reduce_add_sync(0xffffffffu, of_warp & ~(1u << 31));
+    if (__any_sync(0xffffffffu, of_warp >> 31) || total != (unsigned)kCap) {
       radix_way<ENCODE>(src_keys, src_vals, dst_keys, dst_vals, m, enc, smem, s_red);
       return;
     }
+    unsigned run = __reduce_add_sync(0xffffffffu, lane < warp ? of_warp : 0u) + incl - sum;
 #pragma unroll
     for (int i = 0; i < kWordsPerThread; ++i) {
       if (w0 + i < (unsigned)kWords) s_bins[w0 + i].y = run;
       run = __dp4a(cnt[i], 0x01010101u, run);
     }
     __syncthreads();
-    auto size_of = [&](int j) { return (at[j] >> 16) & 0x3fu; };  // <= 31
-    auto rank_of = [&](int j) { return (at[j] >> 22) & 0x1fu; };
-    auto own_place = [&](int j) { return (at[j] & 0xffffu) + rank_of(j); };
     // (loads and stores are kept in loops of their own: the compiler does not move a load over a store)
+    unsigned second = 0;  // items that are the second of their bin
 #pragma unroll
     for (int j = 0; j < ITEMS; ++j) {
       const unsigned bin = at[j] & 0xffffu, rank = at[j] >> 16;
@@ -327,79 +312,90 @@ struct BlockSort {
       const unsigned pick = 0x4440u | (bin & 3u);
       const unsigned begin = w.y + __byte_perm(w.x * 0x01010100u, 0, pick);  // counters of a word: 31 each at most
       const unsigned size = __byte_perm(w.x, 0, pick);
-      at[j] = begin | (size << 16) | (rank << 22);
-      if (j >= have) at[j] = (begin + rank) | (1u << 16);  // alone
+      at[j] = (begin + rank) | (size << 16);
+      if (rank == 1 && j < have) second |= 1u << j;
     }
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) s_index[at[j] & 0xffffu] = (unsigned short)(first + j * kWarp);
+    V val[!kBeside && VB ? ITEMS : 1];
+    if constexpr (!kBeside && VB != 0 && VB <= 8) load(src_vals, val);  // under way while the order is repaired
+    __syncthreads();
+    // Order inside the bins. The counters are no longer needed: each warp lists the bins it has to sort in its share
+    // of their memory, begin | size << 16.
+    unsigned* list = reinterpret_cast<unsigned*>(s_bins) + warp * kListEntries;
+    unsigned entries = 0;
+    auto sort_listed = [&]() {
+      __syncwarp();
+      for (unsigned e = lane; e < entries; e += kWarp) {
+        const unsigned begin = list[e] & 0xffffu, size = list[e] >> 16;
+        const unsigned short x0 = s_index[begin], x1 = s_index[begin + 1];  // two keys as a rule
+        const UK k0 = s_keys[x0], k1 = s_keys[x1];
+        if (k1 < k0 || (k1 == k0 && x1 < x0)) {
+          s_index[begin] = x1;
+          s_index[begin + 1] = x0;
+        }
+        for (unsigned a = 2; a < size; ++a) {  // insertion of the others
+          const unsigned short x = s_index[begin + a];
+          const UK k = s_keys[x];
+          unsigned c = a;
+          for (; c > 0; --c) {
+            const unsigned short y = s_index[begin + c - 1];
+            const UK ky = s_keys[y];
+            if (ky < k || (ky == k && y < x)) break;
+            s_index[begin + c] = y;
+          }
+          if (c != a) s_index[begin + c] = x;
+        }
+      }
+    };
 #pragma unroll
     for (int j = 0; j < ITEMS; ++j) {
-      const unsigned p = own_place(j);
-      s_win[p] = win[j];
-      if (VB != 0 && size_of(j) > 1) s_pos[p] = (unsigned short)(first + j * kWarp);
-    }
-    __syncthreads();
-    // Order inside the bins, by window: step i compares with the key i ranks on, round and round. Two steps are
-    // taken for all elements at once, so that their loads overlap; few bins hold more than three keys.
-    const bool whole = sizeof(UK) < 8 || shift == 0;  // the window is all of the key that varies
-    unsigned again = 0;
-    auto other = [&](int j, unsigned i) -> unsigned {
-      unsigned q = rank_of(j) + i;
-      q = q >= size_of(j) ? q - size_of(j) : q;
-      return (at[j] & 0xffffu) + q;
-    };
-    auto earlier = [&](int j, unsigned q) -> bool {  // the equal key at place q stays in front of key j
-      return VB != 0 ? (unsigned)s_pos[q] < first + j * kWarp : q < own_place(j);
-    };
-    auto step = [&](int j, unsigned i) {
-      if (i < size_of(j)) {
-        const unsigned q = other(j, i), w = s_win[q];
-        bool below = w < win[j];
-        if (w == win[j]) {
-          if (whole) below = earlier(j, q);
-          else again = 1;
-        }
-        if (below) at[j] += 1u << 27;
+      if (kListEntries < kWarp * ITEMS && entries + kWarp > (unsigned)kListEntries) {
+        sort_listed();
+        __syncwarp();
+        entries = 0;
       }
-    };
+      const bool mine = second >> j & 1u;
+      const unsigned votes = __ballot_sync(0xffffffffu, mine);
+      if (mine) list[entries + __popc(votes & lanemask_lt())] = at[j] - 1u;
+      entries += __popc(votes);
+    }
+    sort_listed();
+    __syncthreads();
+
+    const int out = ((int)m - (int)threadIdx.x + THREADS - 1) / THREADS;  // places j * THREADS + thread, j < out
+    const unsigned short* my_index = s_index + threadIdx.x;
+    UK* to_keys = dst_keys + threadIdx.x;
+    unsigned from[ITEMS];
 #pragma unroll
-    for (int j = 0; j < ITEMS; ++j) step(j, 1);
+    for (int j = 0; j < ITEMS; ++j) from[j] = my_index[j * THREADS];
+    const bool plain = (enc.cmask | enc.dmask) == 0;
+    UK key[ITEMS];
 #pragma unroll
-    for (int j = 0; j < ITEMS; ++j) step(j, 2);
+    for (int j = 0; j < ITEMS; ++j) key[j] = s_keys[from[j]];
+    if (!plain) {
+#pragma unroll
+      for (int j = 0; j < ITEMS; ++j) key[j] = decode_key(key[j], enc);
+    }
 #pragma unroll
     for (int j = 0; j < ITEMS; ++j)
-      for (unsigned i = 3; i < size_of(j); ++i) step(j, i);
-    if (!whole && __syncthreads_or(again)) {  // equal windows: whole keys, then positions
-      UK key[ITEMS];
-      load_keys(key, std::true_type{});
+      if (j < out) to_keys[j * THREADS] = key[j];
+    if constexpr (VB != 0) {
+      if constexpr (!kBeside) {
+        __syncthreads();
+        if constexpr (VB > 8) load(src_vals, val);
+#pragma unroll
+        for (int j = 0; j < ITEMS; ++j) s_vals[first + j * kWarp] = val[j];
+        __syncthreads();
+      }
+      V* to_vals = dst_vals + threadIdx.x;
+      V last[ITEMS];
+#pragma unroll
+      for (int j = 0; j < ITEMS; ++j) last[j] = s_vals[from[j]];
 #pragma unroll
       for (int j = 0; j < ITEMS; ++j)
-        if (size_of(j) > 1) s_keys[own_place(j)] = key[j];
-      __syncthreads();
-#pragma unroll
-      for (int j = 0; j < ITEMS; ++j) {
-        if (size_of(j) > 1) at[j] &= (1u << 27) - 1u;
-        for (unsigned i = 1; i < size_of(j); ++i) {
-          const unsigned q = other(j, i);
-          const UK k = s_keys[q];
-          if (k < key[j] || (k == key[j] && earlier(j, q))) at[j] += 1u << 27;
-        }
-      }
+        if (j < out) to_vals[j * THREADS] = last[j];
     }
-    {
-      UK key[ITEMS];
-      V val[VB ? ITEMS : 1];
-      if constexpr (sizeof(UK) == 8) load_keys(key, std::true_type{});
-      if constexpr (VB != 0) load(src_vals, val, std::false_type{});
-      __syncthreads();
-#pragma unroll
-      for (int j = 0; j < ITEMS; ++j) {
-        const unsigned p = (at[j] & 0xffffu) + (at[j] >> 27);
-        if constexpr (sizeof(UK) == 8) s_keys[p] = key[j];
-        else s_keys[p] = (UK)win[j];
-        if constexpr (VB != 0) s_vals[p] = val[j];
-      }
-    }
-    __syncthreads();
-    write_out(dst_keys, dst_vals, s_keys, s_vals, m, enc);
   }
 };
 
