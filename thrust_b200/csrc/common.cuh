@@ -234,6 +234,30 @@ inline cudaError_t launch_chained(void (*kernel)(P...), unsigned grid, unsigned 
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
+// Shared-memory opt-in and residency (CTAs per SM) of one kernel, asked of the runtime once per
+// device. Tag names the kernel's instantiation: all instantiations share one function-pointer type.
+template <typename Tag, typename Kernel>
+int resident_ctas(Kernel kernel, int threads, size_t smem, int* per_sm) {
+  static int cached[64] = {};  // 0: not asked yet (benign race: the answer is always the same)
+  int dev = 0;
+  TB200_CUDA_TRY(cudaGetDevice(&dev));
+  if (dev < 64 && cached[dev] > 0) { *per_sm = cached[dev]; return TB200_OK; }
+  TB200_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  TB200_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kernel, threads, smem));
+  if (*per_sm < 1) return TB200_ERR_UNSUPPORTED;
+  if (dev < 64) cached[dev] = *per_sm;
+  return TB200_OK;
+}
+inline int sm_count_of_device(int* sms) {
+  static int cached[64] = {};
+  int dev = 0;
+  TB200_CUDA_TRY(cudaGetDevice(&dev));
+  if (dev < 64 && cached[dev]) { *sms = cached[dev]; return TB200_OK; }
+  TB200_CUDA_TRY(cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev));
+  if (dev < 64) cached[dev] = *sms;
+  return TB200_OK;
+}
+
 #endif  // __CUDACC__
 
 }  // namespace tb200

@@ -12,6 +12,7 @@
 #include "common.cuh"
 
 #include <mutex>
+#include <type_traits>
 
 namespace tb200 {
 namespace {
@@ -238,6 +239,167 @@ scan_kernel(const T* in, T* out, uint64_t n, T init, TempHeader* hdr,
 }
 
 // ---------------------------------------------------------------------------------------
+// Inputs of which every CTA takes ONE tile: all tiles are in flight at once, so a tile needs no chain of prefixes.
+// Every CTA publishes the sum of its tile and adds up the sums of ALL tiles in front of it itself, one tile per
+// thread: one trip to L2 whatever the number of tiles (a 32-wide chain takes a trip per 32 tiles, and the streaming
+// kernel's ring of five tiles per CTA leaves four SMs in five without work at these sizes). The sums are added in a
+// fixed order, so results do not vary from run to run.
+//   CLUSTER: at most kClusterTiles tiles, one thread-block cluster. The sums travel through distributed shared memory:
+//            nothing in the scratch needs clearing, the scan is a single launch.
+//   else:    tiles are drawn by ticket (a tile only waits for running CTAs) and the sums travel through the scratch.
+// Latency-bound, device time in a replayed graph: 100003 int64 elements 21.4 -> 9.8 us, 1048576 int64 25 -> 16 us,
+// 4194304 float 29 -> 17.5 us (clear and launch included; an empty call measures about 8.5 us this way).
+// ---------------------------------------------------------------------------------------
+constexpr int kClusterTiles = 16;
+
+template <typename T, bool EXCLUSIVE, int K, bool CLUSTER>
+__global__ void __launch_bounds__(kScanThreads, kScanMinCtas)
+scan_wave_kernel(const T* in, T* out, uint64_t n, T init, TempHeader* hdr, TileWords<Words<T>::W>* tiles, int aligned) {
+  constexpr int W = Words<T>::W;
+  constexpr int VEC = 16 / sizeof(T);
+  constexpr int WARP_ITEMS = kWarp * K * VEC;
+  constexpr int TILE = kScanThreads * K * VEC;
+  __shared__ unsigned s_tile;
+  __shared__ T s_warp_total[kScanWarps];
+  __shared__ T s_before[kScanWarps];
+  __shared__ T s_total;  // CLUSTER: the tile's sum, read by the tiles behind it
+
+  unsigned tile;
+  if constexpr (CLUSTER) {
+    tile = blockIdx.x;
+    if (tile == 0 && threadIdx.x == 0) hdr->status = 0;
+  } else {
+    if (threadIdx.x == 0) s_tile = atomicAdd(&hdr->ticket, 1u);
+    __syncthreads();
+    tile = s_tile;
+  }
+  const unsigned warp = threadIdx.x / kWarp;
+  const unsigned lane = lane_id();
+  const uint64_t tile_base = (uint64_t)tile * TILE;
+  const uint64_t warp_base = tile_base + (uint64_t)warp * WARP_ITEMS;
+  const bool full = aligned && tile_base + TILE <= n;
+
+  T x[K][VEC];
+  if (full) {
+    const Vec16<T>* src = reinterpret_cast<const Vec16<T>*>(in + warp_base);
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const Vec16<T> v = src[k * kWarp + lane];
+#pragma unroll
+      for (int j = 0; j < VEC; ++j) x[k][j] = v.v[j];
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+#pragma unroll
+      for (int j = 0; j < VEC; ++j) {
+        const uint64_t i = warp_base + (uint64_t)(k * kWarp + lane) * VEC + j;
+        x[k][j] = i < n ? in[i] : T(0);
+      }
+  }
+
+  // inclusive sums inside each vector, then across the lanes of the warp
+  T excl[K];
+  T carry = T(0);
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+#pragma unroll
+    for (int j = 1; j < VEC; ++j) x[k][j] = x[k][j - 1] + x[k][j];
+    T s = x[k][VEC - 1];
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const T t = __shfl_up_sync(0xffffffffu, s, off);
+      if (lane >= off) s = t + s;
+    }
+    T e = __shfl_up_sync(0xffffffffu, s, 1);
+    if (lane == 0) e = T(0);
+    excl[k] = carry + e;
+    carry = carry + __shfl_sync(0xffffffffu, s, 31);
+  }
+  if (lane == 31) s_warp_total[warp] = carry;
+  __syncthreads();
+  T warp_prefix = T(0), tile_total = T(0);
+#pragma unroll
+  for (int w = 0; w < kScanWarps; ++w) {
+    const T t = s_warp_total[w];
+    if (w < (int)warp) warp_prefix = warp_prefix + t;
+    tile_total = tile_total + t;
+  }
+
+  // the sum of the tile, and thread i's share of what lies in front of it: the sum of tile i
+  T before = T(0);
+  if constexpr (CLUSTER) {
+    if (threadIdx.x == 0) s_total = tile_total;
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (threadIdx.x < tile) {
+      unsigned remote;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(&s_total)), "r"(threadIdx.x));
+      unsigned w[W];
+#pragma unroll
+      for (int i = 0; i < W; ++i)
+        asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(w[i]) : "r"(remote + 4u * i) : "memory");
+      before = Words<T>::unpack(w);
+    }
+  } else {
+    if (threadIdx.x == 0) {
+      unsigned payload[W];
+      Words<T>::pack(tile_total, payload);
+      publish<W>(&tiles[tile], kStateAggregate, payload);
+    }
+    if (threadIdx.x < tile) {
+      unsigned payload[W], polls = 0;
+      bool timed_out = false;
+      while (peek<W>(&tiles[threadIdx.x], payload) == kStateEmpty) {
+        backoff(++polls);
+        if (polls >= kSpinLimit || ((polls & 255u) == 0 && ld_relaxed_s32(&hdr->status) != 0)) {
+          timed_out = true;
+          break;
+        }
+      }
+      if (timed_out) atomicExch(&hdr->status, (int)TB200_ERR_WAIT_TIMEOUT);
+      else before = Words<T>::unpack(payload);
+    }
+  }
+  // add the shares in the order of the tiles (tile <= kScanThreads, so one share per thread is all there is)
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const T o = __shfl_down_sync(0xffffffffu, before, off);
+    if (lane + off < 32) before = before + o;
+  }
+  if (lane == 0) s_before[warp] = before;
+  __syncthreads();
+  T base = init;  // the seed: in front of the first element in both forms
+#pragma unroll
+  for (int w = 0; w < kScanWarps; ++w) base = base + s_before[w];
+  base = base + warp_prefix;
+
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const T p = base + excl[k];
+    Vec16<T> v;
+#pragma unroll
+    for (int j = 0; j < VEC; ++j) {
+      if (EXCLUSIVE) v.v[j] = j == 0 ? p : p + x[k][j - 1];
+      else           v.v[j] = p + x[k][j];
+    }
+    if (full) {
+      reinterpret_cast<Vec16<T>*>(out + warp_base)[k * kWarp + lane] = v;
+    } else {
+#pragma unroll
+      for (int j = 0; j < VEC; ++j) {
+        const uint64_t i = warp_base + (uint64_t)(k * kWarp + lane) * VEC + j;
+        if (i < n) out[i] = v.v[j];
+      }
+    }
+  }
+  if constexpr (CLUSTER) {  // a CTA's shared memory stays until every tile behind it has read its sum
+    asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+  }
+}
+
+// ---------------------------------------------------------------------------------------
 // Streaming variant (16-byte aligned input and output): persistent CTAs, one per SM, each
 // with 16 compute warps and one look-back warp.
 //  * a ring of (park + 2) tiles in shared memory is filled by bulk asynchronous copies
@@ -313,11 +475,11 @@ scan_stream_kernel(const T* in, T* out, uint64_t n, T init, TempHeader* hdr, Til
       mbar_init(&s_resolved[s], 1);
     }
     mbar_init_fence();
-    unsigned first[S];
+    // Ticket after ticket, each drawn when the one before has arrived: drawn in one burst, a CTA's first tiles would be
+    // neighbours, every other CTA's first tile would wait for all of them, and few CTAs would share a short input
+    // (10 M floats 43 -> 25 us, 2^28 floats 409 -> 388 us).
 #pragma unroll
-    for (int s = 0; s < S; ++s) first[s] = atomicAdd(&hdr->ticket, 1u);
-#pragma unroll
-    for (int s = 0; s < S; ++s) start_load(s, first[s]);
+    for (int s = 0; s < S; ++s) start_load(s, atomicAdd(&hdr->ticket, 1u));
     pending = atomicAdd(&hdr->ticket, 1u);
   }
   __syncthreads();
@@ -487,6 +649,44 @@ scan_stream_kernel(const T* in, T* out, uint64_t n, T init, TempHeader* hdr, Til
   }
 }
 
+template <typename T, bool EXCLUSIVE, int K, bool CLUSTER> struct WaveTag {};
+template <typename T, bool EXCLUSIVE> struct StreamTag {};
+
+template <int K, typename T>
+constexpr uint64_t wave_tile() { return (uint64_t)kScanThreads * K * (16 / sizeof(T)); }
+
+// One launch, one tile per CTA: at most kClusterTiles tiles in one cluster, or as many as the GPU holds at once.
+template <typename T, bool EXCLUSIVE, int K, bool CLUSTER>
+int launch_wave(const T* in, T* out, uint64_t n, T init, TempHeader* hdr, TileWords<Words<T>::W>* desc, int aligned,
+                cudaStream_t stream) {
+  auto kernel = scan_wave_kernel<T, EXCLUSIVE, K, CLUSTER>;
+  const unsigned tiles = (unsigned)((n + wave_tile<K, T>() - 1) / wave_tile<K, T>());
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(tiles);
+  cfg.blockDim = dim3(kScanThreads);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr = {};
+  if constexpr (CLUSTER) {
+    if (tiles > 8) {  // more than eight CTAs per cluster are an opt-in
+      static bool allowed[64] = {};  // benign race: the answer is always the same
+      int dev = 0;
+      TB200_CUDA_TRY(cudaGetDevice(&dev));
+      if (dev >= 64 || !allowed[dev]) {
+        TB200_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        if (dev < 64) allowed[dev] = true;
+      }
+    }
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = tiles;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+  }
+  TB200_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, in, out, n, init, hdr, desc, aligned));
+  trace_mark(stream, kTraceScan);
+  return TB200_OK;
+}
+
 template <typename T>
 int launch_scan(void* d_temp, size_t* temp_bytes, const void* d_in, void* d_out, uint64_t n,
                 int exclusive, const void* h_init, cudaStream_t stream) {
@@ -496,14 +696,28 @@ int launch_scan(void* d_temp, size_t* temp_bytes, const void* d_in, void* d_out,
   const uint64_t tiles = (n + TILE - 1) / TILE;
   const uint64_t stream_tiles = (n + STREAM_TILE - 1) / STREAM_TILE;  // the smaller tile sizes the scratch
   const size_t need = kHeaderBytes + (size_t)stream_tiles * sizeof(TileWords<W>);
+  // inputs of one wave of CTAs may take smaller tiles, if the scratch has room for their descriptors
+  const uint64_t small_tiles = (n + wave_tile<4, T>() - 1) / wave_tile<4, T>();
+  const size_t small_need = kHeaderBytes + (size_t)small_tiles * sizeof(TileWords<W>);
   if (d_temp == nullptr) {
-    *temp_bytes = need;
+    *temp_bytes = small_tiles <= (uint64_t)kScanThreads && small_need > need ? small_need : need;
     return TB200_OK;
   }
   if (*temp_bytes < need) return TB200_ERR_TEMP_TOO_SMALL;
   if (reinterpret_cast<uintptr_t>(d_temp) % 256) return TB200_ERR_INVALID_ARGUMENT;
   if (stream_tiles > 0x7fffffffull) return TB200_ERR_UNSUPPORTED;
-  TB200_CUDA_TRY(cudaMemsetAsync(d_temp, 0, need, stream));
+  // One cluster serves up to 1 MiB of input and needs no cleared scratch.
+  const bool cluster = n != 0 && n <= kClusterTiles * wave_tile<8, T>();
+  int sms = 0;
+  {
+    const int rc = sm_count_of_device(&sms);
+    if (rc) return rc;
+  }
+  // One wave: as many tiles as the GPU holds CTAs of that kernel (19 MiB of input on 148 SMs in 64 KiB tiles).
+  const uint64_t resident = (uint64_t)sms * kScanMinCtas < kScanThreads ? (uint64_t)sms * kScanMinCtas : kScanThreads;
+  const bool wave_small = small_tiles <= resident && *temp_bytes >= small_need;
+  const bool wave_large = n <= resident * wave_tile<8, T>();
+  if (!cluster) TB200_CUDA_TRY(cudaMemsetAsync(d_temp, 0, wave_small ? small_need : need, stream));
   if (n == 0) return TB200_OK;
   if (d_in == nullptr || d_out == nullptr) return TB200_ERR_INVALID_ARGUMENT;
 
@@ -514,23 +728,32 @@ int launch_scan(void* d_temp, size_t* temp_bytes, const void* d_in, void* d_out,
   const T* in = static_cast<const T*>(d_in);
   T* out = static_cast<T*>(d_out);
   const bool aligned = ((reinterpret_cast<uintptr_t>(d_in) | reinterpret_cast<uintptr_t>(d_out)) % 16) == 0;
+  auto wave = [&](auto k, auto in_cluster) -> int {
+    constexpr int K = decltype(k)::value;
+    constexpr bool C = decltype(in_cluster)::value;
+    return exclusive ? launch_wave<T, true, K, C>(in, out, n, init, hdr, desc, aligned, stream)
+                     : launch_wave<T, false, K, C>(in, out, n, init, hdr, desc, aligned, stream);
+  };
+  if (cluster) {
+    if (n <= kClusterTiles * wave_tile<2, T>()) return wave(std::integral_constant<int, 2>{}, std::true_type{});
+    return wave(std::integral_constant<int, 8>{}, std::true_type{});
+  }
+  if (wave_small) return wave(std::integral_constant<int, 4>{}, std::false_type{});
+  if (wave_large) return wave(std::integral_constant<int, 8>{}, std::false_type{});
   if (aligned && stream_tiles >= 8) {
-    int dev = 0, sms = 0;
-    TB200_CUDA_TRY(cudaGetDevice(&dev));
-    TB200_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     constexpr int smem = StreamShape<sizeof(T)>::kStages * StreamShape<sizeof(T)>::kTileBytes;
-    auto run = [&](auto kernel) -> int {
-      TB200_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    auto run = [&](auto kernel, auto tag) -> int {
       int per_sm = 0;
-      TB200_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kStreamCta, smem));
-      if (per_sm < 1) return TB200_ERR_UNSUPPORTED;
+      const int rc = resident_ctas<decltype(tag)>(kernel, kStreamCta, smem, &per_sm);
+      if (rc) return rc;
       // one CTA per slot of the GPU: more would only queue behind them
-      const uint64_t resident = (uint64_t)sms * per_sm;
-      const unsigned grid = (unsigned)(stream_tiles < resident ? stream_tiles : resident);
+      const uint64_t slots = (uint64_t)sms * per_sm;
+      const unsigned grid = (unsigned)(stream_tiles < slots ? stream_tiles : slots);
       kernel<<<grid, kStreamCta, smem, stream>>>(in, out, n, init, hdr, desc, (unsigned)stream_tiles);
       return TB200_OK;
     };
-    const int rc = exclusive ? run(scan_stream_kernel<T, true>) : run(scan_stream_kernel<T, false>);
+    const int rc = exclusive ? run(scan_stream_kernel<T, true>, StreamTag<T, true>{})
+                             : run(scan_stream_kernel<T, false>, StreamTag<T, false>{});
     if (rc) return rc;
     trace_mark(stream, kTraceScan);
     return (int)cudaGetLastError();

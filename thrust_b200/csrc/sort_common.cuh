@@ -113,30 +113,6 @@ __device__ __forceinline__ unsigned match_digit(unsigned d) {
   return peers;
 }
 
-// Shared-memory opt-in and residency (CTAs per SM) of one kernel, asked of the runtime once per
-// device. Tag names the kernel's instantiation: all instantiations share one function-pointer type.
-template <typename Tag, typename Kernel>
-int resident_ctas(Kernel kernel, int threads, size_t smem, int* per_sm) {
-  static int cached[64] = {};  // 0: not asked yet (benign race: the answer is always the same)
-  int dev = 0;
-  TB200_CUDA_TRY(cudaGetDevice(&dev));
-  if (dev < 64 && cached[dev] > 0) { *per_sm = cached[dev]; return TB200_OK; }
-  TB200_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  TB200_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kernel, threads, smem));
-  if (*per_sm < 1) return TB200_ERR_UNSUPPORTED;
-  if (dev < 64) cached[dev] = *per_sm;
-  return TB200_OK;
-}
-inline int sm_count_of_device(int* sms) {
-  static int cached[64] = {};
-  int dev = 0;
-  TB200_CUDA_TRY(cudaGetDevice(&dev));
-  if (dev < 64 && cached[dev]) { *sms = cached[dev]; return TB200_OK; }
-  TB200_CUDA_TRY(cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev));
-  if (dev < 64) cached[dev] = *sms;
-  return TB200_OK;
-}
-
 // Copies `bytes` with the whole grid. The source is 256-byte aligned scratch; the destination is the caller's and is
 // written byte by byte when it is not 16-byte aligned.
 __device__ __forceinline__ void copy_back(uint4* __restrict__ dst, const uint4* __restrict__ src, uint64_t bytes) {
