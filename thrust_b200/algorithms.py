@@ -49,6 +49,42 @@ def _temp(nbytes: int, device) -> torch.Tensor:
     return torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device=device)
 
 
+_SLOT = 256  # bytes in front of a scratch of ours: the result of a call lies in the last 16 of them
+
+
+def _workspace(need: int, device, temp: Optional[torch.Tensor]):
+    """(what owns the memory, scratch address, its bytes, address of a 16-byte result slot). The slot lies directly in
+    front of the scratch, so that tb200_read_result fetches it together with the status word; beside a caller's own
+    scratch it is an allocation of its own."""
+    if temp is not None and temp.numel() >= need:
+        slot = torch.empty(16, dtype=torch.uint8, device=device)
+        return (temp, slot), temp.data_ptr(), temp.numel(), slot.data_ptr()
+    block = torch.empty(_SLOT + max(int(need), 256), dtype=torch.uint8, device=device)
+    at = block.data_ptr()
+    return block, at + _SLOT, block.numel() - _SLOT, at + _SLOT - 16
+
+
+class _On:
+    """torch.cuda.device(device), without the two device switches when it is current already."""
+
+    def __init__(self, device: torch.device):
+        self.guard = None if torch.cuda.current_device() == device.index else torch.cuda.device(device)
+
+    def __enter__(self):
+        if self.guard is not None:
+            self.guard.__enter__()
+
+    def __exit__(self, *exc):
+        if self.guard is not None:
+            self.guard.__exit__(*exc)
+
+
+def _result(scratch: int, slot: int, ctype, stream, what: str):
+    value = ctype()
+    capi.check(capi.lib.tb200_read_result(scratch, slot, C.sizeof(ctype), C.byref(value), stream), what)
+    return value.value
+
+
 def _finish(temp: torch.Tensor, stream, what: str, sync: bool) -> None:
     if sync:
         capi.check(capi.lib.tb200_temp_status(C.c_void_p(temp.data_ptr()), stream), what)
@@ -71,7 +107,7 @@ def sort_by_key(keys: torch.Tensor, values: Optional[torch.Tensor] = None, desce
         vptr = values.data_ptr()
     if end_bit is None:
         end_bit = 8 * keys.element_size()
-    with torch.cuda.device(keys.device):
+    with _On(keys.device):
         stream = _stream(keys)
         need = C.c_size_t(0)
         capi.check(capi.lib.tb200_radix_sort(None, C.byref(need), None, None, n, kd, vb, int(descending),
@@ -111,7 +147,7 @@ def _scan(inp: torch.Tensor, out: Optional[torch.Tensor], exclusive: bool, init,
         ctype = {capi.I32: C.c_int32, capi.U32: C.c_uint32, capi.I64: C.c_int64, capi.U64: C.c_uint64,
                  capi.F32: C.c_float, capi.F64: C.c_double}[dt]
         init_buf = ctype(init)
-    with torch.cuda.device(inp.device):
+    with _On(inp.device):
         stream = _stream(inp)
         need = C.c_size_t(0)
         capi.check(capi.lib.tb200_scan(None, C.byref(need), None, None, n, dt, int(exclusive), None, stream),
@@ -156,22 +192,18 @@ def reduce(inp: torch.Tensor, init=None, dtype: Optional[int] = None, out: Optio
     ctype = ctypes_of[dt]
     init_buf = ctype(init) if init is not None else None
     n = inp.numel()
-    if out is None:
-        out = torch.empty(16, dtype=torch.uint8, device=inp.device)
-    with torch.cuda.device(inp.device):
+    with _On(inp.device):
         stream = _stream(inp)
         need = C.c_size_t(0)
         capi.check(capi.lib.tb200_reduce(None, C.byref(need), None, n, dt, None, None, stream), "tb200_reduce(size)")
-        if temp is None or temp.numel() < need.value:
-            temp = _temp(need.value, inp.device)
-        have = C.c_size_t(temp.numel())
-        capi.check(capi.lib.tb200_reduce(C.c_void_p(temp.data_ptr()), C.byref(have),
-                                         C.c_void_p(inp.data_ptr()) if n else None, n, dt,
-                                         C.byref(init_buf) if init_buf is not None else None,
-                                         C.c_void_p(out.data_ptr()), stream), "tb200_reduce")
-        _finish(temp, stream, "tb200_reduce", True)
-    raw = bytes(out.view(torch.uint8)[:C.sizeof(ctype)].cpu().numpy().tobytes())
-    return ctype.from_buffer_copy(raw).value
+        owner, scratch, size, slot = _workspace(need.value, inp.device, temp)
+        if out is not None:
+            slot = out.data_ptr()
+        have = C.c_size_t(size)
+        capi.check(capi.lib.tb200_reduce(scratch, C.byref(have), C.c_void_p(inp.data_ptr()) if n else None, n, dt,
+                                         C.byref(init_buf) if init_buf is not None else None, slot, stream),
+                   "tb200_reduce")
+        return _result(scratch, slot, ctype, stream, "tb200_reduce")
 
 
 def _scan_by_key(keys: torch.Tensor, values: torch.Tensor, out: Optional[torch.Tensor], exclusive: bool, init,
@@ -196,7 +228,7 @@ def _scan_by_key(keys: torch.Tensor, values: torch.Tensor, out: Optional[torch.T
         ctype = {capi.I32: C.c_int32, capi.U32: C.c_uint32, capi.I64: C.c_int64, capi.U64: C.c_uint64,
                  capi.F32: C.c_float, capi.F64: C.c_double}[vd]
         init_buf = ctype(init)
-    with torch.cuda.device(keys.device):
+    with _On(keys.device):
         stream = _stream(keys)
         need = C.c_size_t(0)
         capi.check(capi.lib.tb200_scan_by_key(None, C.byref(need), None, None, None, n, kd, vd, int(exclusive), None,
@@ -243,21 +275,18 @@ def reduce_by_key(keys: torch.Tensor, values: torch.Tensor, keys_out: Optional[t
         keys_out = torch.empty_like(keys)
     if values_out is None:
         values_out = torch.empty_like(values)
-    with torch.cuda.device(keys.device):
+    with _On(keys.device):
         stream = _stream(keys)
-        runs = torch.zeros(1, dtype=torch.int64, device=keys.device)
         need = C.c_size_t(0)
         capi.check(capi.lib.tb200_reduce_by_key(None, C.byref(need), None, None, None, None, None, n, kd, vd,
                                                 stream), "tb200_reduce_by_key(size)")
-        if temp is None or temp.numel() < need.value:
-            temp = _temp(need.value, keys.device)
-        have = C.c_size_t(temp.numel())
+        owner, scratch, size, slot = _workspace(need.value, keys.device, temp)
+        have = C.c_size_t(size)
         capi.check(capi.lib.tb200_reduce_by_key(
-            C.c_void_p(temp.data_ptr()), C.byref(have), C.c_void_p(keys.data_ptr()),
-            C.c_void_p(values.data_ptr()), C.c_void_p(keys_out.data_ptr()), C.c_void_p(values_out.data_ptr()),
-            C.c_void_p(runs.data_ptr()), n, kd, vd, stream), "tb200_reduce_by_key")
-        _finish(temp, stream, "tb200_reduce_by_key", True)
-        return keys_out, values_out, int(runs.item())
+            scratch, C.byref(have), C.c_void_p(keys.data_ptr()), C.c_void_p(values.data_ptr()),
+            C.c_void_p(keys_out.data_ptr()), C.c_void_p(values_out.data_ptr()), slot, n, kd, vd, stream),
+            "tb200_reduce_by_key")
+        return keys_out, values_out, _result(scratch, slot, C.c_int64, stream, "tb200_reduce_by_key")
 
 
 def unique_by_key(keys: torch.Tensor, values: Optional[torch.Tensor] = None, keys_out: Optional[torch.Tensor] = None,
@@ -283,22 +312,19 @@ def unique_by_key(keys: torch.Tensor, values: Optional[torch.Tensor] = None, key
             keys_out = torch.empty_like(keys)
         if values is not None and values_out is None:
             values_out = torch.empty_like(values)
-    with torch.cuda.device(keys.device):
+    with _On(keys.device):
         stream = _stream(keys)
-        count = torch.zeros(1, dtype=torch.int64, device=keys.device)
         need = C.c_size_t(0)
         capi.check(capi.lib.tb200_unique_by_key(None, C.byref(need), None, None, None, None, None, n, kd, vb, stream),
                    "tb200_unique_by_key(size)")
-        if temp is None or temp.numel() < need.value:
-            temp = _temp(need.value, keys.device)
-        have = C.c_size_t(temp.numel())
+        owner, scratch, size, slot = _workspace(need.value, keys.device, temp)
+        have = C.c_size_t(size)
         capi.check(capi.lib.tb200_unique_by_key(
-            C.c_void_p(temp.data_ptr()), C.byref(have), C.c_void_p(keys.data_ptr()),
+            scratch, C.byref(have), C.c_void_p(keys.data_ptr()),
             C.c_void_p(values.data_ptr()) if values is not None else None, C.c_void_p(keys_out.data_ptr()),
-            C.c_void_p(values_out.data_ptr()) if values_out is not None else None, C.c_void_p(count.data_ptr()), n, kd,
-            vb, stream), "tb200_unique_by_key")
-        _finish(temp, stream, "tb200_unique_by_key", True)
-        return keys_out, values_out, int(count.item())
+            C.c_void_p(values_out.data_ptr()) if values_out is not None else None, slot, n, kd, vb, stream),
+            "tb200_unique_by_key")
+        return keys_out, values_out, _result(scratch, slot, C.c_int64, stream, "tb200_unique_by_key")
 
 
 def unique(keys: torch.Tensor, out: Optional[torch.Tensor] = None, key_dtype: Optional[int] = None,
@@ -322,21 +348,17 @@ def copy_flagged(data: torch.Tensor, flags: torch.Tensor, out: Optional[torch.Te
     if out is None:
         out = torch.empty_like(data)
     _check_tensor(out, "out")
-    with torch.cuda.device(data.device):
+    with _On(data.device):
         stream = _stream(data)
-        count = torch.zeros(1, dtype=torch.int64, device=data.device)
         need = C.c_size_t(0)
         capi.check(capi.lib.tb200_copy_flagged(None, C.byref(need), None, None, None, None, n, data.element_size(), fd,
                                                stream), "tb200_copy_flagged(size)")
-        if temp is None or temp.numel() < need.value:
-            temp = _temp(need.value, data.device)
-        have = C.c_size_t(temp.numel())
+        owner, scratch, size, slot = _workspace(need.value, data.device, temp)
+        have = C.c_size_t(size)
         capi.check(capi.lib.tb200_copy_flagged(
-            C.c_void_p(temp.data_ptr()), C.byref(have), C.c_void_p(data.data_ptr()), C.c_void_p(flags.data_ptr()),
-            C.c_void_p(out.data_ptr()), C.c_void_p(count.data_ptr()), n, data.element_size(), fd, stream),
-            "tb200_copy_flagged")
-        _finish(temp, stream, "tb200_copy_flagged", True)
-        return out, int(count.item())
+            scratch, C.byref(have), C.c_void_p(data.data_ptr()), C.c_void_p(flags.data_ptr()),
+            C.c_void_p(out.data_ptr()), slot, n, data.element_size(), fd, stream), "tb200_copy_flagged")
+        return out, _result(scratch, slot, C.c_int64, stream, "tb200_copy_flagged")
 
 
 def histogram_sorted(sorted_data: torch.Tensor, bin_values: torch.Tensor, dtype: Optional[int] = None,
@@ -346,7 +368,7 @@ def histogram_sorted(sorted_data: torch.Tensor, bin_values: torch.Tensor, dtype:
     _check_tensor(bin_values, "bin_values")
     dt = tb200_dtype(sorted_data, dtype)
     counts = torch.empty(bin_values.numel(), dtype=torch.int32, device=sorted_data.device)
-    with torch.cuda.device(sorted_data.device):
+    with _On(sorted_data.device):
         stream = _stream(sorted_data)
         capi.check(capi.lib.tb200_histogram_sorted(C.c_void_p(sorted_data.data_ptr()), sorted_data.numel(), dt,
                                                    C.c_void_p(bin_values.data_ptr()), bin_values.numel(),

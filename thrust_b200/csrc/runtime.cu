@@ -2,6 +2,8 @@
 // pool and the host-buffer entry points (stage in, run the device path, copy out).
 #include "common.cuh"
 
+#include <string.h>
+
 #include <map>
 #include <mutex>
 #include <utility>
@@ -101,11 +103,59 @@ extern "C" const char* tb200_error_string(int code) {
   }
 }
 
+namespace tb200 {
+namespace {
+
+// Pinned landing place of the small read-backs, one per host thread: a copy into pageable memory is staged and waited
+// for by the runtime once more before the stream is (about 5 us a call).
+constexpr size_t kLandingBytes = 512;
+struct Landing {
+  unsigned char* ptr = nullptr;
+  bool tried = false;
+  unsigned char* get() {
+    if (!tried) {
+      tried = true;
+      void* p = nullptr;
+      if (cudaHostAlloc(&p, kLandingBytes, cudaHostAllocPortable) == cudaSuccess) ptr = static_cast<unsigned char*>(p);
+      else (void)cudaGetLastError();
+    }
+    return ptr;
+  }
+  ~Landing() { if (ptr) cudaFreeHost(ptr); }
+};
+thread_local Landing t_landing;
+
+}  // namespace
+}  // namespace tb200
+
 extern "C" int tb200_temp_status(const void* d_temp, tb200_stream_t stream) {
-  if (d_temp == nullptr) return TB200_ERR_INVALID_ARGUMENT;
-  int st = 0;
-  TB200_CUDA_TRY(cudaMemcpyAsync(&st, d_temp, sizeof(int), cudaMemcpyDeviceToHost, stream));
+  return tb200_read_result(d_temp, nullptr, 0, nullptr, stream);
+}
+
+extern "C" int tb200_read_result(const void* d_temp, const void* d_value, size_t value_bytes, void* h_value,
+                                 tb200_stream_t stream) {
+  using namespace tb200;
+  if (d_temp == nullptr || value_bytes > 16 || (value_bytes && (!d_value || !h_value))) return TB200_ERR_INVALID_ARGUMENT;
+  unsigned char pageable[kLandingBytes];
+  unsigned char* land = t_landing.get();
+  if (land == nullptr) land = pageable;
+  const char* temp = static_cast<const char*>(d_temp);
+  const char* value = static_cast<const char*>(d_value);
+  const size_t gap = value_bytes && value < temp ? (size_t)(temp - value) : 0;
+  size_t status_at = 0, value_at = 256;
+  if (gap >= value_bytes && gap != 0 && gap <= 256) {  // value, gap, status word
+    TB200_CUDA_TRY(cudaMemcpyAsync(land, value, gap + sizeof(int), cudaMemcpyDeviceToHost, stream));
+    status_at = gap;
+    value_at = 0;
+  } else {
+    TB200_CUDA_TRY(cudaMemcpyAsync(land, temp, sizeof(int), cudaMemcpyDeviceToHost, stream));
+    if (value_bytes)
+      TB200_CUDA_TRY(cudaMemcpyAsync(land + value_at, value, value_bytes, cudaMemcpyDeviceToHost, stream));
+  }
   TB200_CUDA_TRY(cudaStreamSynchronize(stream));
+  int st = 0;
+  memcpy(&st, land + status_at, sizeof(int));
+  if (value_bytes) memcpy(h_value, land + value_at, value_bytes);
   return st;
 }
 
