@@ -655,6 +655,8 @@ template <typename T, bool EXCLUSIVE> struct StreamTag {};
 template <int K, typename T>
 constexpr uint64_t wave_tile() { return (uint64_t)kScanThreads * K * (16 / sizeof(T)); }
 
+constexpr int kNoCluster = -1000;  // the GPU (or the part of it this process has) holds no cluster of that size
+
 // One launch, one tile per CTA: at most kClusterTiles tiles in one cluster, or as many as the GPU holds at once.
 template <typename T, bool EXCLUSIVE, int K, bool CLUSTER>
 int launch_wave(const T* in, T* out, uint64_t n, T init, TempHeader* hdr, TileWords<Words<T>::W>* desc, int aligned,
@@ -667,20 +669,32 @@ int launch_wave(const T* in, T* out, uint64_t n, T init, TempHeader* hdr, TileWo
   cfg.stream = stream;
   cudaLaunchAttribute attr = {};
   if constexpr (CLUSTER) {
-    if (tiles > 8) {  // more than eight CTAs per cluster are an opt-in
-      static bool allowed[64] = {};  // benign race: the answer is always the same
-      int dev = 0;
-      TB200_CUDA_TRY(cudaGetDevice(&dev));
-      if (dev >= 64 || !allowed[dev]) {
-        TB200_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        if (dev < 64) allowed[dev] = true;
-      }
-    }
     attr.id = cudaLaunchAttributeClusterDimension;
     attr.val.clusterDim.x = tiles;
     attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
+    if (tiles > 8) {
+      // More than eight CTAs per cluster are an opt-in, and need room for all of them in one part of the GPU: asked
+      // once per device (benign race: the answer is always the same).
+      static signed char answer[64] = {};  // 0: not asked, 1: fits, -1: does not
+      int dev = 0;
+      TB200_CUDA_TRY(cudaGetDevice(&dev));
+      signed char fits = dev < 64 ? answer[dev] : 0;
+      if (fits == 0) {
+        TB200_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        cudaLaunchConfig_t largest = cfg;
+        largest.gridDim = dim3(kClusterTiles);
+        cudaLaunchAttribute of = attr;
+        of.val.clusterDim.x = kClusterTiles;
+        largest.attrs = &of;
+        int clusters = 0;
+        fits = cudaOccupancyMaxActiveClusters(&clusters, kernel, &largest) == cudaSuccess && clusters > 0 ? 1 : -1;
+        (void)cudaGetLastError();
+        if (dev < 64) answer[dev] = fits;
+      }
+      if (fits < 0) return kNoCluster;
+    }
   }
   TB200_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, in, out, n, init, hdr, desc, aligned));
   trace_mark(stream, kTraceScan);
@@ -717,9 +731,7 @@ int launch_scan(void* d_temp, size_t* temp_bytes, const void* d_in, void* d_out,
   const uint64_t resident = (uint64_t)sms * kScanMinCtas < kScanThreads ? (uint64_t)sms * kScanMinCtas : kScanThreads;
   const bool wave_small = small_tiles <= resident && *temp_bytes >= small_need;
   const bool wave_large = n <= resident * wave_tile<8, T>();
-  if (!cluster) TB200_CUDA_TRY(cudaMemsetAsync(d_temp, 0, wave_small ? small_need : need, stream));
-  if (n == 0) return TB200_OK;
-  if (d_in == nullptr || d_out == nullptr) return TB200_ERR_INVALID_ARGUMENT;
+  if (n != 0 && (d_in == nullptr || d_out == nullptr)) return TB200_ERR_INVALID_ARGUMENT;
 
   T init = T(0);
   if (h_init) init = *static_cast<const T*>(h_init);
@@ -735,9 +747,12 @@ int launch_scan(void* d_temp, size_t* temp_bytes, const void* d_in, void* d_out,
                      : launch_wave<T, false, K, C>(in, out, n, init, hdr, desc, aligned, stream);
   };
   if (cluster) {
-    if (n <= kClusterTiles * wave_tile<2, T>()) return wave(std::integral_constant<int, 2>{}, std::true_type{});
-    return wave(std::integral_constant<int, 8>{}, std::true_type{});
+    const int rc = n <= kClusterTiles * wave_tile<2, T>() ? wave(std::integral_constant<int, 2>{}, std::true_type{})
+                                                          : wave(std::integral_constant<int, 8>{}, std::true_type{});
+    if (rc != kNoCluster) return rc;
   }
+  TB200_CUDA_TRY(cudaMemsetAsync(d_temp, 0, wave_small ? small_need : need, stream));
+  if (n == 0) return TB200_OK;
   if (wave_small) return wave(std::integral_constant<int, 4>{}, std::false_type{});
   if (wave_large) return wave(std::integral_constant<int, 8>{}, std::false_type{});
   if (aligned && stream_tiles >= 8) {
