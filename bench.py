@@ -271,8 +271,8 @@ def bench_others(dev, peak):
             bool((torch.bincount((k & 0xFFFF).to(torch.int64), minlength=1 << 16) ==
                   torch.bincount((k0 & 0xFFFF).to(torch.int64), minlength=1 << 16)).all())
     entry("sort_i32_2^25", lambda: tb.sort(k, sync=False, temp=temp), lambda: k.copy_(k0), n, "Gkeys/s", 48.0 * n,
-          "4 passes x (2 reads + 1 write) x 4 B = 48 B/key", verify=c1_ok, moved_bytes=36.0 * n,
-          moved_note="one histogram read + 4 passes x (1 read + 1 write) x 4 B = 36 B/key")
+          "4 passes x (2 reads + 1 write) x 4 B = 48 B/key", verify=c1_ok, moved_bytes=28.0 * n,
+          moved_note="one read for the bucket counts + 2 passes and the tile sort x (1 read + 1 write) x 4 B = 28 B/key")
     del k, k0, temp
 
     # C2: scans over 2^30 elements
@@ -405,8 +405,8 @@ def bench_others(dev, peak):
     entry("sort_by_key_u64_u32_2^28", lambda: tb.sort_by_key(k, v, key_dtype=capi.U64, sync=False, temp=temp),
           lambda: (k.copy_(k0), v.copy_(v0)), n, "Gkeys/s", 256.0 * n,
           "8 passes x (3 x 8 B key + 2 x 4 B value) = 256 B/pair",
-          verify=lambda: _sorted_pairs_ok(k0, v0, k, v, _u64_order), moved_bytes=200.0 * n,
-          moved_note="one histogram read (8 B) + 8 passes x (1 read + 1 write) x 12 B = 200 B/pair")
+          verify=lambda: _sorted_pairs_ok(k0, v0, k, v, _u64_order), moved_bytes=80.0 * n,
+          moved_note="one read for the bucket counts (8 B) + 2 passes and the tile sort x (1 read + 1 write) x 12 B = 80 B/pair")
     del k, v, k0, v0
 
     # C4: (float32, int32) pairs, low entropy
@@ -624,26 +624,41 @@ def main():
 
     # dominant kernel: one onesweep radix pass (trace kind 2) over this rank's pairs. At N > 1 the
     # passes run over the received pairs (about n of them), so n is used for every launch.
-    # (the last 8 radix passes of a step: at N > 1 the splitter sample is sorted first, with tiny passes)
-    pass_ms = [ms for tr in trace_ms for ms in [m for kind, m in tr if kind == 2][-8:]]
+    # (the last 8 radix passes of a step: at N > 1 the splitter sample is sorted first, with tiny passes; a sort with a
+    # bucket plan enqueues eight as well, of which those behind the second return at once and are left out)
+    last8 = [[m for kind, m in tr if kind == 2][-8:] for tr in trace_ms]
+    pass_ms = [m for ms in last8 for m in ms if m > 0.1 * max(ms)]
+    passes = len(pass_ms) / max(len(trace_ms), 1)
     avg_pass = sum(pass_ms) / max(len(pass_ms), 1)
     pass_bytes = n * 2.0 * (8 + 4)
     achieved = pass_bytes / (avg_pass * 1e-3) / 1e9 if avg_pass > 0 else 0.0
     tpp = traffic_per_pair()
-    def last_sort(tr):  # launches of the last local sort of a step: histogram, passes, copy-back
+    def last_sort(tr):  # launches of the last local sort of a step: plan, histogram, passes, tiles or copy-back
         idx = [i for i, (kind, _) in enumerate(tr) if kind == 1]
-        return tr[idx[-1]:] if idx else []
-    sort_ms = [sum(ms for kind, ms in last_sort(tr) if kind in (1, 2, 3)) for tr in trace_ms]
-    whole = (256.0 * n) / (sum(sort_ms) / max(len(sort_ms), 1) * 1e-3) / 1e9 if sort_ms and sort_ms[0] > 0 else None
+        if not idx:
+            return []
+        first = idx[-1]
+        while first > 0 and tr[first - 1][0] == 14:
+            first -= 1
+        return tr[first:]
+    sort_ms = [sum(ms for kind, ms in last_sort(tr) if kind in (1, 2, 3, 14, 15)) for tr in trace_ms]
+    planned = any(kind == 15 for tr in trace_ms for kind, _ in tr) and passes < 8
+    # bytes per pair: the keys once for the counts, one read and one write per pass, and with a bucket plan one more
+    # read and write of the tile sort
+    moved = 8 + 24 * passes + (24 if planned else 0)
+    whole = (moved * n) / (sum(sort_ms) / max(len(sort_ms), 1) * 1e-3) / 1e9 if sort_ms and sort_ms[0] > 0 else None
+    tile_ms = [ms for tr in trace_ms for kind, ms in last_sort(tr) if kind == 15] if planned else []
     roofline = {
         "bound": "hbm", "kernel": "onesweep_kernel<u64 key, 4-byte value>", "achieved": achieved, "peak": peak,
         "unit": "GB/s", "frac": achieved / peak, "peak_source": peak_kind,
         "traffic": None if tpp is None else tpp * n, "algorithmic_bytes_per_launch": pass_bytes,
-        "avg_launch_ms": avg_pass, "launches_timed": len(pass_ms),
-        "whole_sort_3touch": {
-            "bytes_per_pair": 256, "model": "8 passes x (2 reads + 1 write of an 8 B key, 1 read + 1 write of a 4 B value)",
+        "avg_launch_ms": avg_pass, "launches_timed": len(pass_ms), "passes_per_sort": passes,
+        "tile_sort_ms": sum(tile_ms) / len(tile_ms) if tile_ms else None,
+        "whole_sort_moved": {
+            "bytes_per_pair": moved,
+            "model": "keys read once for the counts + 1 read and 1 write of every pair per radix pass and in the tile sort",
             "achieved": whole, "frac": None if whole is None else whole / peak,
-            "note": "local sort only (histogram + 8 passes + copy-back launches)",
+            "note": "local sort only (its launches, summed)",
         },
     }
     launches = sum(len(tr) for tr in trace_ms)
