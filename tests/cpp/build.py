@@ -1,8 +1,8 @@
 """Build the C++ boundary test (Thrust custom system over the C ABI) and the small C++ timing
 program of the policy path for sm_100a.
 
-Output: tests/cpp/bin/test_system, bench_system and test_sample_sort (the C entry point of the
-sharded sort called from C++), linked against thrust_b200/libthrust_b200.so by relative rpath. Uses the CUDA toolkit's Thrust headers.
+Output: tests/cpp/bin/test_system, bench_system, test_sample_sort (the C entry point of the
+sharded sort called from C++) and test_tile_sort (the shared-memory sort in each of its shapes), linked against thrust_b200/libthrust_b200.so by relative rpath. Uses the CUDA toolkit's Thrust headers.
 """
 import os
 import subprocess
@@ -12,12 +12,14 @@ from pathlib import Path
 HERE = Path(__file__).resolve().parent
 ROOT = HERE.parent.parent
 LIBDIR = ROOT / "thrust_b200"
-PROGRAMS = ("test_system", "bench_system", "test_sample_sort")
+PROGRAMS = ("test_system", "bench_system", "test_sample_sort", "test_tile_sort")
 
 
 def _build_one(name: str, force: bool) -> Path:
     src, out = HERE / f"{name}.cu", HERE / "bin" / name
     deps = [src, ROOT / "include" / "thrust_b200" / "system.h", ROOT / "include" / "thrust_b200.h"]
+    if name == "test_tile_sort":  # includes device headers of the library
+        deps += (LIBDIR / "csrc").glob("*.cuh")
     if not force and out.exists() and out.stat().st_mtime >= max(d.stat().st_mtime for d in deps):
         return out
     out.parent.mkdir(exist_ok=True)

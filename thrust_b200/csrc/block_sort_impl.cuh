@@ -33,7 +33,9 @@ struct BlockSort {
   static constexpr int kCap = THREADS * ITEMS;
   // Bins in words of four 8-bit counters; the padding behind the last element counts in bins of its own, so that no
   // step but the first load and the last store asks whether an element exists. A word sits beside its scan.
-  static constexpr int kPadBins = 128;
+  // in_front() adds the counters of a word in one byte, so three of them have to stay below 256: a real bin holds fewer
+  // than kCrowd, a padding bin up to kCap / kPadBins (136 of 17408 elements in 128 bins would be too many).
+  static constexpr int kPadBins = 3 * (kCap / 128) < 256 ? 128 : 256;
   static constexpr int kRealWords = BINS / 4;
   static constexpr int kWords = kRealWords + kPadBins / 4;
   static constexpr int kWordsPerThread = ((kWords + THREADS - 1) / THREADS) | 1;
@@ -55,7 +57,18 @@ struct BlockSort {
   static_assert(kListEntries >= 2 * kWarp, "a list is emptied when the next keys might not fit");
   static constexpr int kRedWords = 3 * kWarps;  // static shared words the caller provides
   static_assert(kCap < 65536, "places are 16-bit");
-  static_assert(kCap / kPadBins < 256 && THREADS % kPadBins == 0, "the padding's counters are 8 bits wide too");
+  static_assert(THREADS % kPadBins == 0 && kCap % kPadBins == 0, "the padding fills its bins evenly");
+  static_assert(3 * (kCap / kPadBins) < 256 && 3 * (kCrowd - 1) < 256, "sums of three counters are 8 bits wide too");
+
+  __host__ __device__ static unsigned pad_bin(unsigned thread) { return BINS + thread % kPadBins; }
+  // Elements that the counters of `word` in front of counter `b` hold.
+  __host__ __device__ static unsigned in_front(unsigned word, unsigned b) {
+#ifdef __CUDA_ARCH__
+    return __byte_perm(word * 0x01010100u, 0, 0x4440u | b);
+#else
+    return (word * 0x01010100u >> (8 * b)) & 0xffu;
+#endif
+  }
 
   // Exclusive scan of one number per thread.
   __device__ static unsigned scan_threads(unsigned x, unsigned* s_red) {
@@ -257,13 +270,13 @@ struct BlockSort {
     int narrow = max(0, 32 - __clz((int)(mx - mn)) - kBinBits);
     if ((mx >> narrow) - (mn >> narrow) >= (unsigned)BINS) ++narrow;
     const unsigned bin0 = mn >> narrow;
-    const unsigned pad_bin = BINS + threadIdx.x % kPadBins;
+    const unsigned pad = pad_bin(threadIdx.x);
 
     unsigned at[ITEMS];  // bin | rank inside the bin << 16
 #pragma unroll
     for (int j = 0; j < ITEMS; ++j) {
       unsigned bin = (win[j] >> narrow) - bin0;
-      if (j >= have) bin = pad_bin;
+      if (j >= have) bin = pad;
       const unsigned sh = (bin & 3u) * 8u;
       at[j] = atomicAdd(&s_bins[bin >> 2].x, 1u << sh);
       at[j] = bin | (((at[j] >> sh) & 0xffu) << 16);
@@ -309,9 +322,8 @@ struct BlockSort {
     for (int j = 0; j < ITEMS; ++j) {
       const unsigned bin = at[j] & 0xffffu, rank = at[j] >> 16;
       const uint2 w = s_bins[bin >> 2];
-      const unsigned pick = 0x4440u | (bin & 3u);
-      const unsigned begin = w.y + __byte_perm(w.x * 0x01010100u, 0, pick);  // counters of a word: 31 each at most
-      const unsigned size = __byte_perm(w.x, 0, pick);
+      const unsigned begin = w.y + in_front(w.x, bin & 3u);
+      const unsigned size = __byte_perm(w.x, 0, 0x4440u | (bin & 3u));
       at[j] = (begin + rank) | (size << 16);
       if (rank == 1 && j < have) second |= 1u << j;
     }

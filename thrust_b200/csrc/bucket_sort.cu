@@ -408,15 +408,6 @@ bucket_sort_kernel(UK* main_keys, UK* alt_keys, typename ValueOf<VB>::type* main
   }
 }
 
-// Threads, items per thread, bins and CTAs per SM of the tile sort, smallest capacity first. The tile sort is bound by
-// shared-memory wavefronts and issue slots together (about 9 us per tile of 4096 pairs and CTA, 2 CTAs per SM, 2^28
-// (u64,u32) pairs: 2.0 ms at 3.2 TB/s); 8192 bins (0.4 % slower), 768 x 6 (3 % slower), 512 x 9 three times per SM with
-// 40 registers (5 % slower on 64-bit keys) and 384 x 12 (equal) were tried.
-template <int SIZE> struct TileShape;
-template <> struct TileShape<0> { static constexpr int kThreads = 512, kItems = 9, kBins = 16384, kMinCtas = 2; };
-template <> struct TileShape<1> { static constexpr int kThreads = 1024, kItems = 9, kBins = 16384, kMinCtas = 1; };
-template <> struct TileShape<2> { static constexpr int kThreads = 1024, kItems = 17, kBins = 16384, kMinCtas = 1; };
-
 template <int SIZE> constexpr uint64_t tile_capacity() { return (uint64_t)TileShape<SIZE>::kThreads * TileShape<SIZE>::kItems; }
 
 // The shape whose capacity leaves five standard deviations above the mean of 2^16 evenly filled buckets; -1: none.
