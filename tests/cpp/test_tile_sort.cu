@@ -93,7 +93,7 @@ bool tiles_ok(const char* name) {
   std::mt19937_64 rng(SIZE + 10 * VB);
   // first the small tiles: they meet whatever the shared memory held before
   std::vector<unsigned> sizes = {1, 2, 600, 3000, 31, 33, 6499, 6500, 6526, 6527, cap / 2, cap - 1, cap, 0, 1, cap / 3, cap, 5};
-  for (int i = 0; i < 40; ++i) sizes.push_back((unsigned)(rng() % (cap + 1)));
+  for (int i = 0; i < 60; ++i) sizes.push_back((unsigned)(rng() % (cap + 1)));
   for (unsigned& m : sizes) m = std::min(m, cap);
   std::vector<unsigned> begin(1, 0u);
   for (unsigned m : sizes) begin.push_back(begin.back() + m);
@@ -108,8 +108,15 @@ bool tiles_ok(const char* name) {
       const UK mask = bits < 8 * (int)sizeof(UK) ? (UK)(((UK)1 << bits) - 1) : (UK)~(UK)0;
       for (unsigned i = begin[t]; i < begin[t + 1]; ++i) {
         const UK r = (UK)rng();
-        const UK x = t % 4 == 3 ? (UK)(r % 37) << (bits - 8)        // crowded bins: the radix way
-                   : t % 4 == 2 ? (UK)(r % (mask / 3 * 2)) : r;    // a range that is no power of two
+        const UK step = mask / 3 / (UK)(sizes[t] + 1) + 1;
+        UK x = r;
+        switch (t % 7) {
+          case 2: x = (UK)(r % (mask / 3 * 2)); break;                         // a range that is no power of two
+          case 3: x = (UK)(r % 37) << (bits - 8); break;                       // many copies: counters overflow
+          case 4: x = (UK)(r % (sizes[t] / 5 + 1)) * step; break;              // five copies of every key
+          case 5: x = (UK)(r % (sizes[t] / 30 + 1)) * (30 * step); break;      // thirty
+          case 6: x = (UK)(r % (sizes[t] / 40 + 1)) * (40 * step) + (UK)(rng() % 3); break;  // three keys to a bin
+        }
         k[i] = high | (x & mask);
       }
     }

@@ -84,3 +84,58 @@ def test_bucket_plan_value_widths(cuda_device, dtype, vbytes):
         capi.check(capi.lib.tb200_temp_status(C.c_void_p(temp.data_ptr()), stream), "status")
         assert to_host(a, dtype).tobytes() == k[order].tobytes(), cut
         assert to_host(b, np.uint8).tobytes() == v[order].tobytes(), cut
+
+
+def _copies(n, copies, dtype, device):
+    g = torch.Generator(device=device)
+    g.manual_seed(n + copies)
+    info = torch.iinfo(dtype)
+    values = torch.randint(info.min, info.max, (max(1, n // copies),), dtype=dtype, device=device, generator=g)
+    return values[torch.randint(0, values.numel(), (n,), device=device, generator=g)]
+
+
+@pytest.mark.parametrize("copies", [2, 5, 16, 60, 150, 400])
+@pytest.mark.parametrize("dtype", [torch.int32, torch.int64])
+def test_keys_with_copies(cuda_device, dtype, copies):
+    for n in (3000, 9000, 700001, 5000011):
+        k = _copies(n, copies, dtype, cuda_device)
+        v = torch.arange(n, dtype=torch.int32, device=cuda_device)
+        want, order = torch.sort(k, stable=True, descending=n == 9000)
+        keys = k.clone()
+        tb.sort(keys, descending=n == 9000)
+        assert torch.equal(keys, want), (n, "keys only")
+        tb.sort_by_key(k, v, descending=n == 9000)
+        assert torch.equal(k, want), n
+        assert torch.equal(v, order.to(torch.int32)), (n, "values (stability)")
+
+
+@pytest.mark.parametrize("dtype", [torch.int64])
+def test_keys_with_copies_are_not_slower_than_byte_wise(cuda_device, dtype):
+    """Copies crowd the bins of the tile sort. A scratch without the plan's 512 KiB gives the byte-wise sort."""
+    n = 1 << 24
+    size = torch.empty(0, dtype=dtype).element_size()
+    code = {4: capi.I32, 8: capi.I64}[size]
+    stream = C.c_void_p(torch.cuda.current_stream(cuda_device).cuda_stream)
+    args = (n, code, 4, 0, 0, 8 * size, stream)
+    need = C.c_size_t(0)
+    capi.check(capi.lib.tb200_radix_sort(None, C.byref(need), None, None, *args), "size")
+    temp = torch.empty(need.value, dtype=torch.uint8, device=cuda_device)
+
+    def device_time(k0, scratch):
+        k, v = k0.clone(), torch.arange(n, dtype=torch.int32, device=cuda_device)
+        times = []
+        for _ in range(6):
+            k.copy_(k0)
+            begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda._sleep(200000)  # the launches are enqueued meanwhile
+            begin.record()
+            capi.check(capi.lib.tb200_radix_sort(C.c_void_p(temp.data_ptr()), C.byref(C.c_size_t(scratch)),
+                                                 C.c_void_p(k.data_ptr()), C.c_void_p(v.data_ptr()), *args), "sort")
+            end.record()
+            end.synchronize()
+            times.append(begin.elapsed_time(end))
+        return min(times)
+
+    for copies in (4, 16, 40, 100):
+        k0 = _copies(n, copies, dtype, cuda_device)
+        assert device_time(k0, need.value) < 1.15 * device_time(k0, need.value - (1 << 19)), copies
