@@ -109,7 +109,7 @@ def test_keys_with_copies(cuda_device, dtype, copies):
         assert torch.equal(v, order.to(torch.int32)), (n, "values (stability)")
 
 
-@pytest.mark.parametrize("dtype", [torch.int64])
+@pytest.mark.parametrize("dtype", [torch.int32, torch.int64])
 def test_keys_with_copies_are_not_slower_than_byte_wise(cuda_device, dtype):
     """Copies crowd the bins of the tile sort. A scratch without the plan's 512 KiB gives the byte-wise sort."""
     n = 1 << 24

@@ -6,7 +6,8 @@
 // shared memory (block_sort_impl.cuh), finishes the sort. 64-bit pairs move three times instead of eight.
 //
 //   bucket_prepare_kernel  clears the scratch; one CTA samples 8192 keys for their common prefix and for buckets
-//                          that are clearly too large (heavy duplicates): then nothing further is spent on the plan
+//                          that are clearly too large (heavy duplicates), another one 32-bit keys for copies: then
+//                          nothing further is spent on the plan
 //   bucket_count_kernel    counts all 2^B buckets exactly in shared memory, 16 bits each. A key outside the sampled
 //                          window is not counted and a counter that overflows loses 65535 or 65536, so the sum
 //                          equals n exactly if every count is right. The last CTA decides: buckets of the top eight
@@ -33,6 +34,7 @@ constexpr uint64_t kTwoPassMin = 1ull << 22;
 struct BucketScratch {
   unsigned count[1 << kMaxBucketBits];
   unsigned tile_begin[(1 << kMaxBucketBits) + 8];
+  unsigned copies;  // the keys have copies: no plan
 };
 
 template <typename UK>
@@ -40,33 +42,16 @@ __device__ __forceinline__ bool in_window(UK k, unsigned window_bits, unsigned l
   return window_bits >= 8 * sizeof(UK) || (unsigned long long)(k >> window_bits) == prefix;
 }
 
+// This thread's samples of part `part` of `parts` of the keys: groups of 16 bytes, evenly spread with a jitter (single keys
+// would cost a sector each: one CTA fetches about two sectors per cycle).
 template <typename UK>
-__global__ void __launch_bounds__(kCountThreads)
-bucket_prepare_kernel(const UK* __restrict__ keys, uint64_t n, Encoding enc, SortCtl* ctl, uint64_t clear_bytes,
-                      BucketScratch* scratch, int min_bits, int max_bits, unsigned capacity, int aligned) {
-  chain_begin();
-  constexpr uint64_t kCtlBytes = align_up(sizeof(SortCtl), 256);
-  char* base = reinterpret_cast<char*>(ctl);
-  const uint4 zero = make_uint4(0, 0, 0, 0);
-  if (blockIdx.x != 0) {  // look-back descriptors and bucket counts
-    const uint64_t stride = (uint64_t)(gridDim.x - 1) * kCountThreads;
-    const uint64_t tid = (uint64_t)(blockIdx.x - 1) * kCountThreads + threadIdx.x;
-    uint4* desc = reinterpret_cast<uint4*>(base + kCtlBytes);
-    for (uint64_t i = tid; i < (clear_bytes - kCtlBytes) / 16; i += stride) desc[i] = zero;
-    uint4* count = reinterpret_cast<uint4*>(scratch->count);
-    for (uint64_t i = tid; i < (uint64_t)(1 << max_bits) / 4; i += stride) count[i] = zero;
-    return;
-  }
-  __shared__ unsigned s_cell[4096];
-  __shared__ unsigned s_diff[2], s_most;
-  // Samples: groups of 16 bytes, evenly spread with a jitter (single keys would cost a sector each: one CTA fetches
-  // about two sectors per cycle).
+__device__ __forceinline__ void load_samples(const UK* __restrict__ keys, uint64_t n, int aligned, unsigned part,
+                                             unsigned parts, UK (&key)[kSamples / kCountThreads]) {
   constexpr int VEC = 16 / sizeof(UK), GROUPS = kSamples / kCountThreads / VEC;
-  const uint64_t step = n / kSamples;  // n >= kSamples
-  UK key[kSamples / kCountThreads];
+  const uint64_t step = n / (kSamples * parts);  // n >= kSamples * parts
 #pragma unroll
   for (int i = 0; i < GROUPS; ++i) {
-    const unsigned s = i * kCountThreads + threadIdx.x;
+    const unsigned s = (part * GROUPS + i) * kCountThreads + threadIdx.x;
     const unsigned long long room = step < 0xffffffffull ? step : 0xffffffffull;
     const unsigned long long jitter = (unsigned long long)(s * 2654435761u) * room >> 32;  // < step
     const uint64_t at = (s * step + jitter) * VEC;
@@ -79,6 +64,88 @@ bucket_prepare_kernel(const UK* __restrict__ keys, uint64_t n, Encoding enc, Sor
       for (int e = 0; e < VEC; ++e) key[i * VEC + e] = keys[at + e];
     }
   }
+}
+
+// Two passes and the tile sort of 32-bit keys save a sixth of the byte-wise sort's time, and lose a third if the keys have
+// copies, because crowded tiles take longer and are more (2^25 keys: 599 us byte-wise; 517 us with the plan if all are
+// distinct, 794 us with 16 copies of each). So there is no plan when sampled keys are met again: c copies of each of n / c
+// keys give c 2^25 / n pairs among 8192 samples. Where that is too few, four times as many are looked at, and those kept
+// whose hash ends in two zeros: four times the pairs. (A key that finds its two cells taken by others is not kept, nor is
+// the key 0.) Neighbours in one group of 16 bytes are counted apart: sorted keys would meet there by chance. A CTA of its
+// own does this: behind the other one's work it took 4 us of the sort.
+template <typename UK>
+__device__ void look_for_copies(const UK* __restrict__ keys, uint64_t n, int aligned, BucketScratch* scratch,
+                                unsigned* s_seen) {
+  constexpr int VEC = 16 / sizeof(UK);
+  __shared__ unsigned s_again, s_beside;
+  constexpr int kMine = kSamples / kCountThreads, kParts = 4;
+  const unsigned parts = n < (1ull << 26) ? 1 : kParts;
+  UK key[kParts][kMine];
+#pragma unroll
+  for (int p = 0; p < kParts; ++p)
+    if (p < (int)parts) load_samples(keys, n, aligned, p, parts, key[p]);
+  for (int i = threadIdx.x; i < kSamples; i += kCountThreads) s_seen[i] = 0;  // sampled keys by their hash, 0: free
+  if (threadIdx.x == 0) s_again = s_beside = 0;
+  __syncthreads();
+  unsigned again = 0, beside = 0;
+#pragma unroll
+  for (int p = 0; p < kParts; ++p) {
+    if (p >= (int)parts) break;
+    unsigned look = 0, hash[kMine], old[kMine];
+#pragma unroll
+    for (int i = 0; i < kMine; ++i) {
+      hash[i] = (unsigned)key[p][i] * 2654435761u;
+      if (i % VEC != 0 && key[p][i] == key[p][i % VEC != 0 ? i - 1 : i]) ++beside;
+      else if ((hash[i] >> 17 & (parts - 1)) == 0) look |= 1u << i;
+    }
+#pragma unroll
+    for (int probe = 0; probe < 2; ++probe) {  // the keys of a thread side by side
+#pragma unroll
+      for (int i = 0; i < kMine; ++i)
+        if (look >> i & 1u) old[i] = atomicCAS(&s_seen[((hash[i] >> 19) + probe) % kSamples], 0u, (unsigned)key[p][i]);
+#pragma unroll
+      for (int i = 0; i < kMine; ++i) {
+        if ((look >> i & 1u) && (old[i] == 0 || old[i] == (unsigned)key[p][i])) {
+          again += old[i] != 0;
+          look &= ~(1u << i);
+        }
+      }
+    }
+  }
+  again = __reduce_add_sync(0xffffffffu, again);
+  beside = __reduce_add_sync(0xffffffffu, beside);
+  if (lane_id() == 0 && again) atomicAdd(&s_again, again);
+  if (lane_id() == 0 && beside) atomicAdd(&s_beside, beside);
+  __syncthreads();
+  if (threadIdx.x == 0) scratch->copies = s_again >= 2 || s_beside >= kSamples / 4 * parts;
+}
+
+template <typename UK>
+__global__ void __launch_bounds__(kCountThreads)
+bucket_prepare_kernel(const UK* __restrict__ keys, uint64_t n, Encoding enc, SortCtl* ctl, uint64_t clear_bytes,
+                      BucketScratch* scratch, int min_bits, int max_bits, unsigned capacity, int aligned) {
+  chain_begin();
+  constexpr uint64_t kCtlBytes = align_up(sizeof(SortCtl), 256);
+  char* base = reinterpret_cast<char*>(ctl);
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  __shared__ unsigned s_cell[sizeof(UK) == 4 ? kSamples : 4096];
+  const bool ask_copies = sizeof(UK) == 4 && n >= kTwoPassMin;
+  const unsigned clear_from = ask_copies ? 2 : 1;  // CTAs in front of those that clear
+  if (blockIdx.x >= clear_from) {  // look-back descriptors and bucket counts
+    const uint64_t stride = (uint64_t)(gridDim.x - clear_from) * kCountThreads;
+    const uint64_t tid = (uint64_t)(blockIdx.x - clear_from) * kCountThreads + threadIdx.x;
+    uint4* desc = reinterpret_cast<uint4*>(base + kCtlBytes);
+    for (uint64_t i = tid; i < (clear_bytes - kCtlBytes) / 16; i += stride) desc[i] = zero;
+    uint4* count = reinterpret_cast<uint4*>(scratch->count);
+    for (uint64_t i = tid; i < (uint64_t)(1 << max_bits) / 4; i += stride) count[i] = zero;
+    return;
+  }
+  if (blockIdx.x == 1) return look_for_copies(keys, n, aligned, scratch, s_cell);
+  if (!ask_copies && threadIdx.x == 0) scratch->copies = 0;
+  __shared__ unsigned s_diff[2], s_most;
+  UK key[kSamples / kCountThreads];
+  const uint64_t step = n / kSamples;
+  load_samples(keys, n, aligned, 0, 1, key);
   const UK ref = encode_key(keys[0], enc);
   for (uint64_t i = threadIdx.x; i < kCtlBytes / 16; i += kCountThreads) reinterpret_cast<uint4*>(base)[i] = zero;
   for (int i = threadIdx.x; i < 4096; i += kCountThreads) s_cell[i] = 0;
@@ -319,7 +386,7 @@ bucket_count_kernel(const UK* __restrict__ keys, uint64_t n, Encoding enc, SortC
   extern __shared__ __align__(16) unsigned s_mem[];  // 2^(bucket_bits - 1) words, two counters each
   __shared__ unsigned s_last;
   chain_begin();
-  if (!ctl->window_ok) return;
+  if (!ctl->window_ok || scratch->copies) return;
   const unsigned window_bits = ctl->window_bits;
   const int bucket_bits = (int)ctl->bucket_bits;
   const unsigned long long prefix = ctl->window_prefix;
@@ -443,10 +510,10 @@ int plan(SortCtl* ctl, size_t clear_bytes, BucketScratch* scratch, const UK* key
   const int min_bits = min_bucket_bits(n, capacity), max_bits = kMaxBucketBits;
   const uint64_t vecs = (clear_bytes + (sizeof(unsigned) << max_bits)) / 16;
   const int aligned = reinterpret_cast<uintptr_t>(keys) % 16 == 0;
-  const uint64_t want = 2 + vecs / (4 * kCountThreads);
-  TB200_CUDA_TRY(launch_chained(bucket_prepare_kernel<UK>, (unsigned)(want < (uint64_t)sms ? want : (uint64_t)sms),
-                                kCountThreads, 0, stream, keys, n, enc, ctl, (uint64_t)clear_bytes, scratch, min_bits,
-                                max_bits, (unsigned)capacity, aligned));
+  const uint64_t want = 3 + vecs / (4 * kCountThreads);  // two CTAs at most look at the keys, the others clear
+  const unsigned grid = (unsigned)(want < (uint64_t)sms ? want : (uint64_t)(sms < 3 ? 3 : sms));
+  TB200_CUDA_TRY(launch_chained(bucket_prepare_kernel<UK>, grid, kCountThreads, 0, stream, keys, n, enc, ctl,
+                                (uint64_t)clear_bytes, scratch, min_bits, max_bits, (unsigned)capacity, aligned));
   trace_mark(stream, kTraceSortPlan);
   auto kernel = bucket_count_kernel<UK>;
   constexpr size_t kMaxSmem = sizeof(uint16_t) << kMaxBucketBits;
