@@ -57,3 +57,40 @@ def test_scan_with_a_scratch_for_the_large_tiles_only(cuda_device):
         capi.check(capi.lib.tb200_temp_status(C.c_void_p(temp.data_ptr()), stream), "status")
         want = torch.cumsum(x, 0, dtype=torch.int32)
         assert torch.equal(out, want - x if exclusive else want)
+
+
+@pytest.mark.parametrize("offset,roundings", [(0, 2), (1, 4)])  # the streaming kernel; pointers that are not aligned
+@pytest.mark.parametrize("exclusive", [False, True])
+def test_float_prefixes_are_not_rounded_tile_by_tile(cuda_device, exclusive, offset, roundings):
+    """Whole numbers below 256: the sums inside a tile are exact (below 2^24), and so is a prefix that is carried in 64
+    bits. What is left is the rounding of the prefix to a float and of each addition behind it: prefix + element in the
+    streaming kernel, prefix + warp + lane + element in the other. Each is at most 2^-24 of a partial sum, and partial sums
+    of positive numbers do not exceed the result by more than these roundings."""
+    n = (1 << 27) + 5
+    g = torch.Generator(device=cuda_device)
+    g.manual_seed(12)
+    x = torch.randint(0, 256, (n + offset,), dtype=torch.int32, device=cuda_device, generator=g)[offset:]
+    f = torch.empty(n + offset, dtype=torch.float32, device=cuda_device)[offset:]
+    f.copy_(x)
+    out = torch.empty(n + offset, dtype=torch.float32, device=cuda_device)[offset:]
+    want = torch.cumsum(x, 0, dtype=torch.int64) + 1000
+    if exclusive:
+        want -= x
+        tb.exclusive_scan(f, out, init=1000.0)
+    else:
+        f[0] += 1000
+        tb.inclusive_scan(f, out)
+    error = ((out.double() - want.double()).abs() / want.double()).max().item()
+    assert error <= roundings * 2.0**-24 * (1 + 2.0**-20)
+
+
+def test_float_scan_beyond_the_largest_float(cuda_device):
+    """A prefix that passes the largest float is an infinity for everything behind it, as if it were carried as a float."""
+    n = 1 << 24
+    x = torch.zeros(n, dtype=torch.float32, device=cuda_device)
+    x[1000], x[2_000_000], x[9_000_000] = 3e38, 3e38, -3e38
+    got = tb.inclusive_scan(x)
+    assert got[999] == 0 and got[1000] == 3e38 and got[1_999_999] == 3e38
+    assert torch.isinf(got[2_000_000:9_000_000]).all() and torch.isinf(got[-1])
+    x[5] = float("nan")
+    assert torch.isnan(tb.inclusive_scan(x)[5:]).all()

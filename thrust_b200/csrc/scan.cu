@@ -51,15 +51,52 @@ struct Words {
   }
 };
 
+// What a descriptor of the look-back chain carries: the sum of a tile, or of everything up to its end.
+template <typename T>
+struct Link {
+  static constexpr int W = Words<T>::W;
+  using Sum = T;
+  __device__ static void publish(TileWords<W>* d, unsigned state, Sum x) {
+    unsigned payload[W];
+    Words<T>::pack(x, payload);
+    tb200::publish<W>(d, state, payload);
+  }
+  __device__ static unsigned peek(const TileWords<W>* d, Sum& x) {
+    unsigned payload[W];
+    const unsigned state = tb200::peek<W>(d, payload);
+    x = Words<T>::unpack(payload);
+    return state;
+  }
+  __device__ static Sum settle(Sum x) { return x; }
+};
+// Sums of floats travel in 64 bits: a prefix is the end of a chain of one addition per tile, and every one of them would
+// round it (2^28 whole numbers, 26215 tiles: errors of up to 24 times 2^-24 of the result, two at most this way; random
+// numbers: 1.1e-6 of the norm, 1.1e-7 this way). The state
+// takes the two lowest bits of the word, so a descriptor stays as small as a float's. A sum beyond the floats becomes the
+// infinity that it would have become as a float.
+template <>
+struct Link<float> {
+  using Sum = double;
+  __device__ static void publish(TileWords<1>* d, unsigned state, Sum x) {
+    st_relaxed_u64(&d->w[0], (__builtin_bit_cast(unsigned long long, x) & ~3ull) | state);
+  }
+  __device__ static unsigned peek(const TileWords<1>* d, Sum& x) {
+    const unsigned long long w = ld_relaxed_u64(&d->w[0]);
+    x = __builtin_bit_cast(double, w & ~3ull);
+    return (unsigned)w & 3u;
+  }
+  __device__ static Sum settle(Sum x) { return isinf((float)x) ? (Sum)(float)x : x; }
+};
+
 // Warp 0 walks back over predecessor descriptors, 32 * kLookSlots at a time (kLookSlots
 // per lane, all loads in flight together), until it meets one that carries a full prefix.
 // Returns the sum of everything before `tile`.
 constexpr int kLookSlots = 1;
 template <typename T>
-__device__ T lookback_sum(const TileWords<Words<T>::W>* tiles, unsigned tile, int* status) {
-  constexpr int W = Words<T>::W;
+__device__ typename Link<T>::Sum lookback_sum(const TileWords<Words<T>::W>* tiles, unsigned tile, int* status) {
+  using Sum = typename Link<T>::Sum;
   const unsigned lane = lane_id();
-  T acc = T(0);
+  Sum acc = Sum(0);
   long long base = (long long)tile - 1;
   bool timed_out = false;
   while (true) {
@@ -67,19 +104,20 @@ __device__ T lookback_sum(const TileWords<Words<T>::W>* tiles, unsigned tile, in
     // back. All loads are issued first; slots are then consumed nearest first and the
     // walk stops at the first prefix, so descriptors behind it are never waited for.
     unsigned st[kLookSlots];
-    unsigned payload[kLookSlots][W];
+    Sum found_sum[kLookSlots];
 #pragma unroll
     for (int s = 0; s < kLookSlots; ++s) {
       const long long idx = base - 32 * s - lane;
       st[s] = kStatePrefix;
-      if (idx >= 0) st[s] = peek<W>(&tiles[idx], payload[s]);
+      found_sum[s] = Sum(0);
+      if (idx >= 0) st[s] = Link<T>::peek(&tiles[idx], found_sum[s]);
     }
     bool found = false;
 #pragma unroll
     for (int s = 0; s < kLookSlots; ++s) {
       if (found) break;
       const long long idx = base - 32 * s - lane;
-      T v = T(0);
+      Sum v = Sum(0);
       if (idx >= 0) {
         unsigned polls = 0;
         while (st[s] == kStateEmpty) {
@@ -89,17 +127,17 @@ __device__ T lookback_sum(const TileWords<Words<T>::W>* tiles, unsigned tile, in
             st[s] = kStatePrefix;
             break;
           }
-          st[s] = peek<W>(&tiles[idx], payload[s]);
+          st[s] = Link<T>::peek(&tiles[idx], found_sum[s]);
         }
-        v = timed_out ? T(0) : Words<T>::unpack(payload[s]);
+        v = timed_out ? Sum(0) : found_sum[s];
       }
       const unsigned pm = __ballot_sync(0xffffffffu, st[s] == kStatePrefix);
       const unsigned first = pm ? (unsigned)(__ffs(pm) - 1) : 31u;
-      if (lane > first) v = T(0);
+      if (lane > first) v = Sum(0);
       // far predecessors (high lanes) are summed before near ones
 #pragma unroll
       for (int off = 1; off < 32; off <<= 1) {
-        T o = __shfl_down_sync(0xffffffffu, v, off);
+        Sum o = __shfl_down_sync(0xffffffffu, v, off);
         if (lane + off < 32) v = o + v;
       }
       v = __shfl_sync(0xffffffffu, v, 0);
@@ -110,14 +148,13 @@ __device__ T lookback_sum(const TileWords<Words<T>::W>* tiles, unsigned tile, in
     base -= 32 * kLookSlots;
   }
   if (__any_sync(0xffffffffu, timed_out) && lane == 0) atomicExch(status, (int)TB200_ERR_WAIT_TIMEOUT);
-  return acc;
+  return Link<T>::settle(acc);
 }
 
 template <typename T, bool EXCLUSIVE, bool ALIGNED>
 __global__ void __launch_bounds__(kScanThreads, kScanMinCtas)
 scan_kernel(const T* in, T* out, uint64_t n, T init, TempHeader* hdr,
             TileWords<Words<T>::W>* tiles) {
-  constexpr int W = Words<T>::W;
   constexpr int VEC = 16 / sizeof(T);
   constexpr int K = kScanVecs;
   constexpr int WARP_ITEMS = kWarp * K * VEC;
@@ -185,26 +222,15 @@ scan_kernel(const T* in, T* out, uint64_t n, T init, TempHeader* hdr,
   }
 
   if (warp == 0) {
-    unsigned payload[W];
-    T prefix;
-    if (tile == 0) {
-      prefix = init;  // the seed: in front of the first element in both forms
-      if (lane == 0) {
-        Words<T>::pack(prefix + tile_total, payload);
-        publish<W>(&tiles[0], kStatePrefix, payload);
-      }
-    } else {
-      if (lane == 0) {
-        Words<T>::pack(tile_total, payload);
-        publish<W>(&tiles[tile], kStateAggregate, payload);
-      }
+    typename Link<T>::Sum prefix = init;  // the seed: in front of the first element in both forms
+    if (tile != 0) {
+      if (lane == 0) Link<T>::publish(&tiles[tile], kStateAggregate, tile_total);
       prefix = lookback_sum<T>(tiles, tile, &hdr->status);
-      if (lane == 0) {
-        Words<T>::pack(prefix + tile_total, payload);
-        publish<W>(&tiles[tile], kStatePrefix, payload);
-      }
     }
-    if (lane == 0) s_tile_prefix = prefix;
+    if (lane == 0) {
+      Link<T>::publish(&tiles[tile], kStatePrefix, Link<T>::settle(prefix + tile_total));
+      s_tile_prefix = (T)prefix;
+    }
   }
   __syncthreads();
   const T base = s_tile_prefix + warp_prefix;
@@ -436,7 +462,6 @@ template <typename T, bool EXCLUSIVE>
 __global__ void __launch_bounds__(kStreamCta, 1)
 scan_stream_kernel(const T* in, T* out, uint64_t n, T init, TempHeader* hdr, TileWords<Words<T>::W>* tiles,
                    unsigned num_tiles) {
-  constexpr int W = Words<T>::W;
   constexpr int VEC = 16 / sizeof(T);
   constexpr int K = StreamShape<sizeof(T)>::kVecs;
   constexpr int kStreamPark = StreamShape<sizeof(T)>::kPark;
@@ -492,17 +517,11 @@ scan_stream_kernel(const T* in, T* out, uint64_t n, T init, TempHeader* hdr, Til
       const unsigned tile = s_look_tile[slot];
       if (tile == kNoTile) break;
       const T total = s_look_total[slot];
-      T prefix;
-      if (tile == 0) {
-        prefix = init;  // the seed: in front of the first element in both forms
-      } else {
-        prefix = lookback_sum<T>(tiles, tile, status);
-      }
+      typename Link<T>::Sum prefix = init;  // the seed: in front of the first element in both forms
+      if (tile != 0) prefix = lookback_sum<T>(tiles, tile, status);
       if (lane == 0) {
-        unsigned payload[W];
-        Words<T>::pack(prefix + total, payload);
-        publish<W>(&tiles[tile], kStatePrefix, payload);
-        s_prefix[slot] = prefix;
+        Link<T>::publish(&tiles[tile], kStatePrefix, Link<T>::settle(prefix + total));
+        s_prefix[slot] = (T)prefix;
         mbar_arrive(&s_resolved[slot]);
       }
       __syncwarp();
@@ -607,11 +626,7 @@ scan_stream_kernel(const T* in, T* out, uint64_t n, T init, TempHeader* hdr, Til
       tile_total = tile_total + t;
     }
     if (threadIdx.x == 0) {
-      if (tile != 0) {
-        unsigned payload[W];
-        Words<T>::pack(tile_total, payload);
-        publish<W>(&tiles[tile], kStateAggregate, payload);
-      }
+      if (tile != 0) Link<T>::publish(&tiles[tile], kStateAggregate, tile_total);
       s_look_tile[slot] = tile;
       s_look_total[slot] = tile_total;
       mbar_arrive(&s_handoff[slot]);
