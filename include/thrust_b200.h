@@ -253,12 +253,15 @@ int tb200_histogram_sorted(const void* d_sorted, uint64_t n, int dtype, const vo
  * (thrust/system/cuda/detail/util.h:113-140, 251-299). */
 int tb200_temp_status(const void* d_temp, tb200_stream_t stream);
 
-/* tb200_temp_status and a result of value_bytes (at most 16) at device address d_value in one go: one copy when the
- * result lies in the 256 bytes in front of d_temp, and one wait for the stream either way. h_value receives the result
- * (undefined when the status is not 0). The reference reads a count back with a copy of its own before it synchronises
- * (thrust/system/cuda/detail/reduce_by_key.h:1049-1052). */
+/* tb200_temp_status and a result of value_bytes (at most 16) at device address d_value with one wait for the stream.
+ * h_value receives the result (undefined when the status is not 0). The reference reads a count back with a copy of its
+ * own before it synchronises (thrust/system/cuda/detail/reduce_by_key.h:1049-1052). */
 int tb200_read_result(const void* d_temp, const void* d_value, size_t value_bytes, void* h_value,
                       tb200_stream_t stream);
+
+/* The same for a result at d_temp - 16, with one copy for both: the caller states that the 16 bytes in front of d_temp
+ * belong to the same allocation. */
+int tb200_read_result_in_front(const void* d_temp, size_t value_bytes, void* h_value, tb200_stream_t stream);
 
 /* Self-test of the bounded-wait convention every kernel here follows: launches one warp that
  * polls a flag nothing ever sets, for at most limit_polls polls (1 .. 2^20), and returns the

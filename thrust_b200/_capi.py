@@ -55,6 +55,7 @@ def _load() -> C.CDLL:
         "tb200_histogram_sorted": ([vp, u64, i32, vp, u32, vp, vp], i32),
         "tb200_temp_status": ([vp, vp], i32),
         "tb200_read_result": ([vp, vp, sz, vp, vp], i32),
+        "tb200_read_result_in_front": ([vp, sz, vp, vp], i32),
         "tb200_selftest_wait_timeout": ([u32, vp], i32),
         "tb200_trace_begin": ([vp], i32),
         "tb200_trace_end": ([C.POINTER(C.c_float), C.POINTER(C.c_int), i32], i32),
@@ -77,7 +78,7 @@ lib = _load()
 
 EXPORTS = [
     "tb200_version", "tb200_error_string", "tb200_radix_sort", "tb200_partition", "tb200_partition_count", "tb200_partition_scatter", "tb200_partition_ties", "tb200_partition_count_ties", "tb200_partition_scatter_ties", "tb200_gather_segments", "tb200_radix_sort_begin", "tb200_radix_sort_finish", "tb200_scan", "tb200_scan_static", "tb200_scan_static_status", "tb200_reduce_by_key", "tb200_reduce", "tb200_scan_by_key", "tb200_unique_by_key", "tb200_copy_flagged",
-    "tb200_histogram_sorted", "tb200_temp_status", "tb200_read_result", "tb200_selftest_wait_timeout", "tb200_trace_begin", "tb200_trace_end",
+    "tb200_histogram_sorted", "tb200_temp_status", "tb200_read_result", "tb200_read_result_in_front", "tb200_selftest_wait_timeout", "tb200_trace_begin", "tb200_trace_end",
     "tb200_workspace_acquire",
     "tb200_workspace_release", "tb200_workspace_stats", "tb200_workspace_release_all", "tb200_radix_sort_host", "tb200_scan_host",
     "tb200_reduce_by_key_host",

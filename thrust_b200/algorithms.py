@@ -53,15 +53,15 @@ _SLOT = 256  # bytes in front of a scratch of ours: the result of a call lies in
 
 
 def _workspace(need: int, device, temp: Optional[torch.Tensor]):
-    """(what owns the memory, scratch address, its bytes, address of a 16-byte result slot). The slot lies directly in
-    front of the scratch, so that tb200_read_result fetches it together with the status word; beside a caller's own
-    scratch it is an allocation of its own."""
+    """(what owns the memory, scratch address, its bytes, address of a 16-byte result slot, whether the slot lies in the
+    scratch's own block, directly in front of it, where one copy fetches it together with the status word). Beside a
+    caller's own scratch the slot is an allocation of its own."""
     if temp is not None and temp.numel() >= need:
         slot = torch.empty(16, dtype=torch.uint8, device=device)
-        return (temp, slot), temp.data_ptr(), temp.numel(), slot.data_ptr()
+        return (temp, slot), temp.data_ptr(), temp.numel(), slot.data_ptr(), False
     block = torch.empty(_SLOT + max(int(need), 256), dtype=torch.uint8, device=device)
     at = block.data_ptr()
-    return block, at + _SLOT, block.numel() - _SLOT, at + _SLOT - 16
+    return block, at + _SLOT, block.numel() - _SLOT, at + _SLOT - 16, True
 
 
 class _On:
@@ -79,9 +79,12 @@ class _On:
             self.guard.__exit__(*exc)
 
 
-def _result(scratch: int, slot: int, ctype, stream, what: str):
+def _result(scratch: int, slot: int, in_front: bool, ctype, stream, what: str):
     value = ctype()
-    capi.check(capi.lib.tb200_read_result(scratch, slot, C.sizeof(ctype), C.byref(value), stream), what)
+    if in_front:
+        capi.check(capi.lib.tb200_read_result_in_front(scratch, C.sizeof(ctype), C.byref(value), stream), what)
+    else:
+        capi.check(capi.lib.tb200_read_result(scratch, slot, C.sizeof(ctype), C.byref(value), stream), what)
     return value.value
 
 
@@ -196,14 +199,14 @@ def reduce(inp: torch.Tensor, init=None, dtype: Optional[int] = None, out: Optio
         stream = _stream(inp)
         need = C.c_size_t(0)
         capi.check(capi.lib.tb200_reduce(None, C.byref(need), None, n, dt, None, None, stream), "tb200_reduce(size)")
-        owner, scratch, size, slot = _workspace(need.value, inp.device, temp)
+        owner, scratch, size, slot, in_front = _workspace(need.value, inp.device, temp)
         if out is not None:
-            slot = out.data_ptr()
+            slot, in_front = out.data_ptr(), False
         have = C.c_size_t(size)
         capi.check(capi.lib.tb200_reduce(scratch, C.byref(have), C.c_void_p(inp.data_ptr()) if n else None, n, dt,
                                          C.byref(init_buf) if init_buf is not None else None, slot, stream),
                    "tb200_reduce")
-        return _result(scratch, slot, ctype, stream, "tb200_reduce")
+        return _result(scratch, slot, in_front, ctype, stream, "tb200_reduce")
 
 
 def _scan_by_key(keys: torch.Tensor, values: torch.Tensor, out: Optional[torch.Tensor], exclusive: bool, init,
@@ -280,13 +283,13 @@ def reduce_by_key(keys: torch.Tensor, values: torch.Tensor, keys_out: Optional[t
         need = C.c_size_t(0)
         capi.check(capi.lib.tb200_reduce_by_key(None, C.byref(need), None, None, None, None, None, n, kd, vd,
                                                 stream), "tb200_reduce_by_key(size)")
-        owner, scratch, size, slot = _workspace(need.value, keys.device, temp)
+        owner, scratch, size, slot, in_front = _workspace(need.value, keys.device, temp)
         have = C.c_size_t(size)
         capi.check(capi.lib.tb200_reduce_by_key(
             scratch, C.byref(have), C.c_void_p(keys.data_ptr()), C.c_void_p(values.data_ptr()),
             C.c_void_p(keys_out.data_ptr()), C.c_void_p(values_out.data_ptr()), slot, n, kd, vd, stream),
             "tb200_reduce_by_key")
-        return keys_out, values_out, _result(scratch, slot, C.c_int64, stream, "tb200_reduce_by_key")
+        return keys_out, values_out, _result(scratch, slot, in_front, C.c_int64, stream, "tb200_reduce_by_key")
 
 
 def unique_by_key(keys: torch.Tensor, values: Optional[torch.Tensor] = None, keys_out: Optional[torch.Tensor] = None,
@@ -317,14 +320,14 @@ def unique_by_key(keys: torch.Tensor, values: Optional[torch.Tensor] = None, key
         need = C.c_size_t(0)
         capi.check(capi.lib.tb200_unique_by_key(None, C.byref(need), None, None, None, None, None, n, kd, vb, stream),
                    "tb200_unique_by_key(size)")
-        owner, scratch, size, slot = _workspace(need.value, keys.device, temp)
+        owner, scratch, size, slot, in_front = _workspace(need.value, keys.device, temp)
         have = C.c_size_t(size)
         capi.check(capi.lib.tb200_unique_by_key(
             scratch, C.byref(have), C.c_void_p(keys.data_ptr()),
             C.c_void_p(values.data_ptr()) if values is not None else None, C.c_void_p(keys_out.data_ptr()),
             C.c_void_p(values_out.data_ptr()) if values_out is not None else None, slot, n, kd, vb, stream),
             "tb200_unique_by_key")
-        return keys_out, values_out, _result(scratch, slot, C.c_int64, stream, "tb200_unique_by_key")
+        return keys_out, values_out, _result(scratch, slot, in_front, C.c_int64, stream, "tb200_unique_by_key")
 
 
 def unique(keys: torch.Tensor, out: Optional[torch.Tensor] = None, key_dtype: Optional[int] = None,
@@ -353,12 +356,12 @@ def copy_flagged(data: torch.Tensor, flags: torch.Tensor, out: Optional[torch.Te
         need = C.c_size_t(0)
         capi.check(capi.lib.tb200_copy_flagged(None, C.byref(need), None, None, None, None, n, data.element_size(), fd,
                                                stream), "tb200_copy_flagged(size)")
-        owner, scratch, size, slot = _workspace(need.value, data.device, temp)
+        owner, scratch, size, slot, in_front = _workspace(need.value, data.device, temp)
         have = C.c_size_t(size)
         capi.check(capi.lib.tb200_copy_flagged(
             scratch, C.byref(have), C.c_void_p(data.data_ptr()), C.c_void_p(flags.data_ptr()),
             C.c_void_p(out.data_ptr()), slot, n, data.element_size(), fd, stream), "tb200_copy_flagged")
-        return out, _result(scratch, slot, C.c_int64, stream, "tb200_copy_flagged")
+        return out, _result(scratch, slot, in_front, C.c_int64, stream, "tb200_copy_flagged")
 
 
 def histogram_sorted(sorted_data: torch.Tensor, bin_values: torch.Tensor, dtype: Optional[int] = None,

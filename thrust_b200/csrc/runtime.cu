@@ -108,7 +108,7 @@ namespace {
 
 // Pinned landing place of the small read-backs, one per host thread: a copy into pageable memory is staged and waited
 // for by the runtime once more before the stream is (about 5 us a call).
-constexpr size_t kLandingBytes = 512;
+constexpr size_t kLandingBytes = 64;
 struct Landing {
   unsigned char* ptr = nullptr;
   bool tried = false;
@@ -125,6 +125,27 @@ struct Landing {
 };
 thread_local Landing t_landing;
 
+// Copies the pieces one behind the other to `out` and waits for the stream.
+struct Piece {
+  const void* from;
+  size_t bytes;
+};
+int fetch(const Piece* piece, int pieces, unsigned char* out, cudaStream_t stream) {
+  unsigned char pageable[kLandingBytes];
+  unsigned char* land = t_landing.get();
+  if (land == nullptr) land = pageable;
+  cudaError_t err = cudaSuccess;
+  size_t at = 0;
+  for (int i = 0; i < pieces && err == cudaSuccess; ++i) {
+    err = cudaMemcpyAsync(land + at, piece[i].from, piece[i].bytes, cudaMemcpyDeviceToHost, stream);
+    at += piece[i].bytes;
+  }
+  const cudaError_t waited = cudaStreamSynchronize(stream);  // after an error too: an earlier piece may be on its way
+  if (err == cudaSuccess) err = waited;
+  if (err == cudaSuccess) memcpy(out, land, at);
+  return (int)err;
+}
+
 }  // namespace
 }  // namespace tb200
 
@@ -136,27 +157,28 @@ extern "C" int tb200_read_result(const void* d_temp, const void* d_value, size_t
                                  tb200_stream_t stream) {
   using namespace tb200;
   if (d_temp == nullptr || value_bytes > 16 || (value_bytes && (!d_value || !h_value))) return TB200_ERR_INVALID_ARGUMENT;
-  unsigned char pageable[kLandingBytes];
-  unsigned char* land = t_landing.get();
-  if (land == nullptr) land = pageable;
-  const char* temp = static_cast<const char*>(d_temp);
-  const char* value = static_cast<const char*>(d_value);
-  const size_t gap = value_bytes && value < temp ? (size_t)(temp - value) : 0;
-  size_t status_at = 0, value_at = 256;
-  if (gap >= value_bytes && gap != 0 && gap <= 256) {  // value, gap, status word
-    TB200_CUDA_TRY(cudaMemcpyAsync(land, value, gap + sizeof(int), cudaMemcpyDeviceToHost, stream));
-    status_at = gap;
-    value_at = 0;
-  } else {
-    TB200_CUDA_TRY(cudaMemcpyAsync(land, temp, sizeof(int), cudaMemcpyDeviceToHost, stream));
-    if (value_bytes)
-      TB200_CUDA_TRY(cudaMemcpyAsync(land + value_at, value, value_bytes, cudaMemcpyDeviceToHost, stream));
-  }
-  TB200_CUDA_TRY(cudaStreamSynchronize(stream));
-  int st = 0;
-  memcpy(&st, land + status_at, sizeof(int));
-  if (value_bytes) memcpy(h_value, land + value_at, value_bytes);
-  return st;
+  // two copies: that the result lies close to the scratch does not make them one allocation
+  const Piece piece[2] = {{d_temp, sizeof(int)}, {d_value, value_bytes}};
+  unsigned char got[sizeof(int) + 16];
+  const int rc = fetch(piece, value_bytes ? 2 : 1, got, stream);
+  if (rc) return rc;
+  int status = 0;
+  memcpy(&status, got, sizeof(int));
+  if (value_bytes) memcpy(h_value, got + sizeof(int), value_bytes);
+  return status;
+}
+
+extern "C" int tb200_read_result_in_front(const void* d_temp, size_t value_bytes, void* h_value, tb200_stream_t stream) {
+  using namespace tb200;
+  if (d_temp == nullptr || value_bytes > 16 || (value_bytes && !h_value)) return TB200_ERR_INVALID_ARGUMENT;
+  const Piece piece = {static_cast<const char*>(d_temp) - 16, 16 + sizeof(int)};
+  unsigned char got[16 + sizeof(int)];
+  const int rc = fetch(&piece, 1, got, stream);
+  if (rc) return rc;
+  int status = 0;
+  memcpy(&status, got + 16, sizeof(int));
+  if (value_bytes) memcpy(h_value, got, value_bytes);
+  return status;
 }
 
 extern "C" int tb200_workspace_acquire(size_t bytes, tb200_stream_t stream, void** d_ptr) {
