@@ -59,13 +59,14 @@ def test_scan_with_a_scratch_for_the_large_tiles_only(cuda_device):
         assert torch.equal(out, want - x if exclusive else want)
 
 
-@pytest.mark.parametrize("offset,roundings", [(0, 2), (1, 4)])  # the streaming kernel; pointers that are not aligned
+@pytest.mark.parametrize("offset,roundings", [(0, 7), (1, 9)])  # the streaming kernel; pointers that are not aligned
 @pytest.mark.parametrize("exclusive", [False, True])
 def test_float_prefixes_are_not_rounded_tile_by_tile(cuda_device, exclusive, offset, roundings):
-    """Whole numbers below 256: the sums inside a tile are exact (below 2^24), and so is a prefix that is carried in 64
-    bits. What is left is the rounding of the prefix to a float and of each addition behind it: prefix + element in the
-    streaming kernel, prefix + warp + lane + element in the other. Each is at most 2^-24 of a partial sum, and partial sums
-    of positive numbers do not exceed the result by more than these roundings."""
+    """Whole numbers below 256: the sums inside a tile are exact (below 2^24), and so are additions to a prefix that is
+    carried in 64 bits. What is left is at most five roundings of the sums of up to 32 tiles that join the prefix together
+    (a tree), the rounding of the prefix to a float, and that of each addition behind it: prefix + element in the streaming
+    kernel, prefix + warp + lane + element in the other. Each is at most 2^-24 of a partial sum, and partial sums of
+    positive numbers do not exceed the result by more than these roundings."""
     n = (1 << 27) + 5
     g = torch.Generator(device=cuda_device)
     g.manual_seed(12)
@@ -81,7 +82,7 @@ def test_float_prefixes_are_not_rounded_tile_by_tile(cuda_device, exclusive, off
         f[0] += 1000
         tb.inclusive_scan(f, out)
     error = ((out.double() - want.double()).abs() / want.double()).max().item()
-    assert error <= roundings * 2.0**-24 * (1 + 2.0**-20)
+    assert error <= roundings * 2.0**-24 * (1 + 2.0**-19)
 
 
 def test_float_scan_beyond_the_largest_float(cuda_device):
