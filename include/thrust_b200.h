@@ -291,7 +291,7 @@ int tb200_trace_end(float* ms, int* kinds, int capacity);
  * back once the caller has ENQUEUED its last use (the block is only handed to later work on the
  * same stream, which runs after it). tb200_workspace_stats reports how many device allocations
  * the pool has made since the library was loaded and how many bytes it holds;
- * tb200_workspace_release_all frees everything (no lease may be outstanding). */
+ * tb200_workspace_release_all frees everything (no lease may be outstanding), the pinned page of the read-backs with it. */
 int tb200_workspace_acquire(size_t bytes, tb200_stream_t stream, void** d_ptr);
 int tb200_workspace_release(void* d_ptr);
 int tb200_workspace_stats(uint64_t* device_allocations, uint64_t* bytes_held);

@@ -61,3 +61,31 @@ assert lib.tb200_read_result_in_front(None, C.c_size_t(8), C.byref(got), None) !
 assert lib.tb200_read_result_in_front(C.c_void_p(scratch), C.c_size_t(17), C.byref(got), None) != 0
 assert lib.tb200_read_result_in_front(C.c_void_p(scratch), C.c_size_t(8), None, None) != 0
 """)
+
+
+def test_short_lived_threads_share_the_pinned_page(tmp_path):
+    """A pinned allocation per thread, freed when it ends, would make every short-lived thread wait for the whole GPU."""
+    _run(tmp_path, """
+put(scratch, C.c_int, 5)
+def work():
+    for _ in range(20): assert lib.tb200_temp_status(C.c_void_p(scratch), None) == 5
+for _ in range(3):
+    threads = [threading.Thread(target=work) for _ in range(8)]
+    for t in threads: t.start()
+    for t in threads: t.join()
+assert count("fake_host_allocs") <= 1 and count("fake_host_frees") == 0, (count("fake_host_allocs"), count("fake_host_frees"))
+lib.tb200_workspace_release_all()
+assert count("fake_host_frees") == count("fake_host_allocs")
+work()
+""")
+
+
+def test_a_failing_copy_is_reported_and_waited_for(tmp_path):
+    _run(tmp_path, """
+put(scratch, C.c_int, 0)
+C.c_int.in_dll(fake, "fake_fail_copy").value = 1  # the second one
+value = scratch - 512 + 64
+assert lib.tb200_read_result(C.c_void_p(scratch), C.c_void_p(value), C.c_size_t(8), C.byref(got), None) == 1
+assert count("fake_syncs") == 1  # the first may still be on its way to the landing place
+assert lib.tb200_temp_status(C.c_void_p(scratch), None) == 0
+""")

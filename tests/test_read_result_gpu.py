@@ -1,5 +1,6 @@
 """tb200_read_result (status word and result by two copies) and tb200_read_result_in_front (by one)."""
 import ctypes as C
+import threading
 
 import pytest
 import torch
@@ -56,3 +57,43 @@ def test_results_beside_a_scratch_of_the_caller(cuda_device):
         assert runs == 33335 and int(sums[:runs].sum()) == x.numel() and torch.equal(keys[:runs], torch.unique(x))
         assert tb.unique_by_key(x, temp=t)[2] == 33335
         assert tb.copy_flagged(x, (x % 2 == 0).to(torch.uint8), temp=t)[1] == int((x % 2 == 0).sum())
+
+
+def test_read_backs_of_many_threads(cuda_device):
+    """Each thread reads results of its own through the slots that all of them share."""
+    wrong = []
+
+    def work(i):
+        stream = torch.cuda.Stream(cuda_device)
+        with torch.cuda.stream(stream):
+            x = torch.full((1000 + i,), i + 1, dtype=torch.int32, device=cuda_device)
+            for _ in range(200):
+                if tb.reduce(x) != (1000 + i) * (i + 1):
+                    wrong.append(i)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(12)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
+
+
+def test_first_read_back_beside_a_capture(cuda_device):
+    """The pinned page is asked for while another thread captures a graph: that must not end the capture."""
+    capi.check(capi.lib.tb200_workspace_release_all(), "release")  # the page too
+    status = torch.full((64,), 7, dtype=torch.int32, device=cuda_device)
+    x = torch.zeros(16, device=cuda_device)
+    stream = torch.cuda.Stream(cuda_device)
+    torch.cuda.synchronize()
+    got = []
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        x.add_(1)
+        t = threading.Thread(target=lambda: got.append(capi.lib.tb200_temp_status(status.data_ptr(), stream.cuda_stream)))
+        t.start()
+        t.join()
+        x.add_(1)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert got == [7] and x[0].item() == 2

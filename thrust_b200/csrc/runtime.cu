@@ -106,24 +106,44 @@ extern "C" const char* tb200_error_string(int code) {
 namespace tb200 {
 namespace {
 
-// Pinned landing place of the small read-backs, one per host thread: a copy into pageable memory is staged and waited
-// for by the runtime once more before the stream is (about 5 us a call).
-constexpr size_t kLandingBytes = 64;
-struct Landing {
-  unsigned char* ptr = nullptr;
-  bool tried = false;
-  unsigned char* get() {
-    if (!tried) {
-      tried = true;
-      void* p = nullptr;
-      if (cudaHostAlloc(&p, kLandingBytes, cudaHostAllocPortable) == cudaSuccess) ptr = static_cast<unsigned char*>(p);
-      else (void)cudaGetLastError();
-    }
-    return ptr;
+// Pinned landing places of the small read-backs: a copy into pageable memory is staged and waited for by the runtime once
+// more before the stream is (about 5 us a call). One page for the process, asked for at the first read-back; a call takes
+// a slot and gives it back. Without a page, or with every slot taken, the copy goes to the caller's stack.
+constexpr size_t kSlotBytes = 64;
+constexpr int kSlots = 64;
+std::mutex g_landing_mutex;
+unsigned char* g_landing_page = nullptr;
+bool g_landing_asked = false;
+unsigned long long g_landing_taken = 0;  // one bit per slot
+
+unsigned char* landing_take() {
+  std::lock_guard<std::mutex> lock(g_landing_mutex);
+  if (!g_landing_asked) {
+    g_landing_asked = true;
+    // another thread may be capturing a graph: the allocation has nothing to do with it and must not end it
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, kSlots * kSlotBytes, cudaHostAllocPortable) == cudaSuccess) g_landing_page = static_cast<unsigned char*>(p);
+    else (void)cudaGetLastError();
+    cudaThreadExchangeStreamCaptureMode(&mode);
   }
-  ~Landing() { if (ptr) cudaFreeHost(ptr); }
-};
-thread_local Landing t_landing;
+  if (g_landing_page == nullptr || ~g_landing_taken == 0) return nullptr;
+  const int slot = __builtin_ctzll(~g_landing_taken);
+  g_landing_taken |= 1ull << slot;
+  return g_landing_page + slot * kSlotBytes;
+}
+void landing_give(unsigned char* p) {
+  std::lock_guard<std::mutex> lock(g_landing_mutex);
+  g_landing_taken &= ~(1ull << ((p - g_landing_page) / kSlotBytes));
+}
+void landing_release() {  // unless a call holds a slot; the next read-back asks again
+  std::lock_guard<std::mutex> lock(g_landing_mutex);
+  if (g_landing_taken != 0) return;
+  if (g_landing_page) cudaFreeHost(g_landing_page);
+  g_landing_page = nullptr;
+  g_landing_asked = false;
+}
 
 // Copies the pieces one behind the other to `out` and waits for the stream.
 struct Piece {
@@ -131,9 +151,9 @@ struct Piece {
   size_t bytes;
 };
 int fetch(const Piece* piece, int pieces, unsigned char* out, cudaStream_t stream) {
-  unsigned char pageable[kLandingBytes];
-  unsigned char* land = t_landing.get();
-  if (land == nullptr) land = pageable;
+  unsigned char pageable[kSlotBytes];
+  unsigned char* slot = landing_take();
+  unsigned char* land = slot ? slot : pageable;
   cudaError_t err = cudaSuccess;
   size_t at = 0;
   for (int i = 0; i < pieces && err == cudaSuccess; ++i) {
@@ -143,6 +163,7 @@ int fetch(const Piece* piece, int pieces, unsigned char* out, cudaStream_t strea
   const cudaError_t waited = cudaStreamSynchronize(stream);  // after an error too: an earlier piece may be on its way
   if (err == cudaSuccess) err = waited;
   if (err == cudaSuccess) memcpy(out, land, at);
+  if (slot && waited == cudaSuccess) landing_give(slot);  // else a copy might still land there
   return (int)err;
 }
 
@@ -261,6 +282,7 @@ extern "C" int tb200_workspace_release_all(void) {
   g_pool_owner.clear();
   g_pool_bytes = 0;
   cudaSetDevice(cur);
+  landing_release();
   return rc;
 }
 
