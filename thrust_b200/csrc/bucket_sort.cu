@@ -191,8 +191,8 @@ bucket_prepare_kernel(const UK* __restrict__ keys, uint64_t n, Encoding enc, Sor
       while (bucket_bits < max_bits && (cell >> (bucket_bits - 12)) > capacity / 2) ++bucket_bits;
       ok = ok && (cell >> (bucket_bits - 12)) <= 2ull * capacity;
     }
-    // 32-bit keys have four byte-wise passes at most: below kTwoPassMin keys only a plan of one pass is worth its count
-    if (sizeof(UK) == 4 && n < kTwoPassMin) ok = ok && s_most <= 16 && n <= (uint64_t)capacity * 237;
+    // below kTwoPassMin 32-bit keys only a plan of one pass is worth its count (bucket_scratch_bytes)
+    if (sizeof(UK) == 4 && n < kTwoPassMin) ok = ok && s_most <= 16;
     ctl->window_ok = ok;
     ctl->bucket_bits = (unsigned)bucket_bits;
     ctl->window_bits = (unsigned)bits;
@@ -478,13 +478,12 @@ bucket_sort_kernel(UK* main_keys, UK* alt_keys, typename ValueOf<VB>::type* main
 template <int SIZE> constexpr uint64_t tile_capacity() { return (uint64_t)TileShape<SIZE>::kThreads * TileShape<SIZE>::kItems; }
 
 // The shape whose capacity leaves five standard deviations above the mean of 2^16 evenly filled buckets; -1: none.
-int tile_size_of(uint64_t n, int key_bytes, int val_bytes) {
+int tile_size_of(uint64_t n, int val_bytes) {
   const uint64_t mean = n >> kMaxBucketBits;
   if (n > (1ull << 30)) return -1;
   if (mean <= 4270) return 0;
   if (mean <= 8700) return 1;
   if (mean <= 16700 && val_bytes <= 8) return 2;
-  (void)key_bytes;
   return -1;
 }
 uint64_t capacity_of(int size) {
@@ -506,7 +505,7 @@ int plan(SortCtl* ctl, size_t clear_bytes, BucketScratch* scratch, const UK* key
   int sms = 0;
   int rc = sm_count_of_device(&sms);
   if (rc) return rc;
-  const uint64_t capacity = capacity_of(tile_size_of(n, sizeof(UK), val_bytes));
+  const uint64_t capacity = capacity_of(tile_size_of(n, val_bytes));
   const int min_bits = min_bucket_bits(n, capacity), max_bits = kMaxBucketBits;
   const uint64_t vecs = (clear_bytes + (sizeof(unsigned) << max_bits)) / 16;
   const int aligned = reinterpret_cast<uintptr_t>(keys) % 16 == 0;
@@ -550,7 +549,7 @@ int finish(const SortCtl* ctl, const BucketScratch* scratch, void* keys, void* k
 template <typename UK, int VB>
 int finish_size(const SortCtl* ctl, const BucketScratch* scratch, void* k, void* ka, void* v, void* va, uint64_t n,
                 const Encoding& enc, cudaStream_t s) {
-  switch (tile_size_of(n, sizeof(UK), VB)) {
+  switch (tile_size_of(n, VB)) {
     case 0: return finish<UK, VB, 0>(ctl, scratch, k, ka, v, va, n, enc, s);
     case 1: return finish<UK, VB, 1>(ctl, scratch, k, ka, v, va, n, enc, s);
     default:
@@ -576,7 +575,12 @@ int finish_vals(int vb, const SortCtl* ctl, const BucketScratch* scratch, void* 
 }  // namespace
 
 size_t bucket_scratch_bytes(uint64_t n, int key_bytes, int val_bytes) {
-  if (key_bytes < 4 || n < kSamples || tile_size_of(n, key_bytes, val_bytes) < 0) return 0;
+  const int size = tile_size_of(n, val_bytes);
+  if (key_bytes < 4 || n < kSamples || size < 0) return 0;
+  // 32-bit keys have four byte-wise passes at most: below kTwoPassMin keys only a plan of one pass is worth its count, and
+  // one pass leaves 256 buckets: more than 237 times a tile's capacity cannot be expected to fit them all (evenly spread
+  // keys: a mean of 237 / 256 of the capacity leaves five standard deviations at 4608).
+  if (key_bytes == 4 && n < kTwoPassMin && n > 237 * capacity_of(size)) return 0;
   return align_up(sizeof(BucketScratch), 256);
 }
 
