@@ -53,11 +53,6 @@ int single_vals(int vb, void* k, void* v, uint64_t n, const Encoding& enc, int* 
 
 }  // namespace
 
-uint64_t block_sort_capacity(int key_bytes, int val_bytes) {
-  (void)key_bytes; (void)val_bytes;
-  return 9216;
-}
-
 int block_sort_single(void* d_keys, void* d_vals, uint64_t n, int key_bytes, int val_bytes, int kind, int descending,
                       int* d_status, cudaStream_t stream) {
   const Encoding enc = make_encoding(key_bytes, kind, descending);

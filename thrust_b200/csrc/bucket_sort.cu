@@ -323,14 +323,7 @@ __device__ void decide(SortCtl* ctl, BucketScratch* scratch, uint64_t n, int buc
   // digit offsets of the passes. Top eight bits: 2^top buckets each, held by four threads.
   __syncthreads();
   {
-    unsigned e = total;
-    e += __shfl_xor_sync(0xffffffffu, e, 1);
-    e += __shfl_xor_sync(0xffffffffu, e, 2);
-    const int p = passes - 1;
-    if ((tid & 3u) == 0) {
-      ctl->offs[p][tid >> 2] = start;
-      ctl->hist[p][tid >> 2] = e;
-    }
+    if ((tid & 3u) == 0) ctl->offs[passes - 1][tid >> 2] = start;
   }
   const unsigned low = 1u << top;
   if (passes == 2) {  // low digit: every 2^top-th bucket, the rows divided among the threads

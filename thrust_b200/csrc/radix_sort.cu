@@ -1,4 +1,7 @@
-// Onesweep LSD radix sort, 8-bit digits, written for sm_100a.
+// Onesweep LSD radix sort, 8-bit digits, written for sm_100a; and the choice between the ways of a sort (sort_impl):
+// whole keys of up to 9216 elements are sorted by one CTA (block_sort.cu); longer whole-key sorts of 4- and 8-byte keys
+// put the bucket plan (bucket_sort.cu) in front and behind: with a plan, passes 1 and 2 below run on its digits, the others
+// return at once, and the tile sort takes the place of step 3. The byte-wise sort:
 //
 //   1. histogram_kernel   one read of the keys builds the digit histogram of EVERY
 //                         pass (shared-memory atomics, then 64-bit global atomics);
@@ -13,7 +16,8 @@
 //                         tiles, reorders keys (and values) through shared memory so
 //                         each digit leaves as one contiguous run, and scatters them.
 //   3. copy_back_kernel   only when an odd number of passes ran (result in the
-//                         alternate buffer); decided on the device, no host sync.
+//                         alternate buffer); decided on the device, no host sync. (Where a
+//                         plan was tried, the tile kernel does this.)
 //
 // Stability: inside a warp keys are ranked in (round, lane) order, which is their
 // order in memory (round j of lane l holds element j*32+l of the warp's slice);
@@ -864,7 +868,7 @@ int sort_impl(void* d_temp, size_t* temp_bytes, void* d_keys, void* d_vals, uint
   // Device time of both: 4096 (i32,i32) pairs 7 against 39 us, 9000 (u64,u32) pairs 14 against 78 us. The line lies
   // where the shared memory of one CTA ends (eight-byte keys with sixteen-byte values).
   const bool whole = begin_bit == 0 && end_bit == 8 * (int)sizeof(UK);
-  if (phase == kPhaseAll && whole && n <= block_sort_capacity(sizeof(UK), VB)) {
+  if (phase == kPhaseAll && whole && n <= kBlockSortCapacity) {
     if (d_keys == nullptr || (VB && d_vals == nullptr)) return TB200_ERR_INVALID_ARGUMENT;
     return block_sort_single(d_keys, d_vals, n, sizeof(UK), VB, kind, descending, &ctl->status, stream);
   }

@@ -159,7 +159,8 @@ __device__ typename Link<T>::Sum lookback_sum(const TileWords<Words<T>::W>* tile
   return Link<T>::settle(acc);
 }
 
-template <typename T, bool EXCLUSIVE, bool ALIGNED>
+// Pointers that are not 16-byte aligned (the streaming kernel's bulk copies need them aligned), above one wave of tiles.
+template <typename T, bool EXCLUSIVE>
 __global__ void __launch_bounds__(kScanThreads, kScanMinCtas)
 scan_kernel(const T* in, T* out, uint64_t n, T init, TempHeader* hdr,
             TileWords<Words<T>::W>* tiles) {
@@ -179,26 +180,15 @@ scan_kernel(const T* in, T* out, uint64_t n, T init, TempHeader* hdr,
   const unsigned lane = lane_id();
   const uint64_t tile_base = (uint64_t)tile * TILE;
   const uint64_t warp_base = tile_base + (uint64_t)warp * WARP_ITEMS;
-  const bool full = tile_base + TILE <= n;
 
   T x[K][VEC];
-  if (ALIGNED && full) {
-    const Vec16<T>* src = reinterpret_cast<const Vec16<T>*>(in + warp_base);
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      Vec16<T> v = src[k * kWarp + lane];
+  for (int k = 0; k < K; ++k)
 #pragma unroll
-      for (int j = 0; j < VEC; ++j) x[k][j] = v.v[j];
+    for (int j = 0; j < VEC; ++j) {
+      const uint64_t i = warp_base + (uint64_t)(k * kWarp + lane) * VEC + j;
+      x[k][j] = i < n ? in[i] : T(0);
     }
-  } else {
-#pragma unroll
-    for (int k = 0; k < K; ++k)
-#pragma unroll
-      for (int j = 0; j < VEC; ++j) {
-        const uint64_t i = warp_base + (uint64_t)(k * kWarp + lane) * VEC + j;
-        x[k][j] = i < n ? in[i] : T(0);
-      }
-  }
 
   // inclusive sums inside each vector, then across the lanes of the warp
   T excl[K];
@@ -243,31 +233,16 @@ scan_kernel(const T* in, T* out, uint64_t n, T init, TempHeader* hdr,
   __syncthreads();
   const T base = s_tile_prefix + warp_prefix;
 
-  if (ALIGNED && full) {
-    Vec16<T>* dst = reinterpret_cast<Vec16<T>*>(out + warp_base);
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const T p = base + excl[k];
-      Vec16<T> v;
+  for (int k = 0; k < K; ++k) {
+    const T p = base + excl[k];
 #pragma unroll
-      for (int j = 0; j < VEC; ++j) {
-        if (EXCLUSIVE) v.v[j] = j == 0 ? p : p + x[k][j - 1];
-        else           v.v[j] = p + x[k][j];
-      }
-      dst[k * kWarp + lane] = v;
-    }
-  } else {
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const T p = base + excl[k];
-#pragma unroll
-      for (int j = 0; j < VEC; ++j) {
-        const uint64_t i = warp_base + (uint64_t)(k * kWarp + lane) * VEC + j;
-        T r;
-        if (EXCLUSIVE) r = j == 0 ? p : p + x[k][j - 1];
-        else           r = p + x[k][j];
-        if (i < n) out[i] = r;
-      }
+    for (int j = 0; j < VEC; ++j) {
+      const uint64_t i = warp_base + (uint64_t)(k * kWarp + lane) * VEC + j;
+      T r;
+      if (EXCLUSIVE) r = j == 0 ? p : p + x[k][j - 1];
+      else           r = p + x[k][j];
+      if (i < n) out[i] = r;
     }
   }
 }
@@ -778,7 +753,7 @@ int launch_scan(void* d_temp, size_t* temp_bytes, const void* d_in, void* d_out,
   if (n == 0) return TB200_OK;
   if (wave_small) return wave(std::integral_constant<int, 4>{}, std::false_type{});
   if (wave_large) return wave(std::integral_constant<int, 8>{}, std::false_type{});
-  if (aligned && stream_tiles >= 8) {
+  if (aligned) {
     constexpr int smem = StreamShape<sizeof(T)>::kStages * StreamShape<sizeof(T)>::kTileBytes;
     auto run = [&](auto kernel, auto tag) -> int {
       int per_sm = 0;
@@ -797,13 +772,8 @@ int launch_scan(void* d_temp, size_t* temp_bytes, const void* d_in, void* d_out,
     return (int)cudaGetLastError();
   }
   const dim3 grid((unsigned)tiles), block(kScanThreads);
-  if (exclusive) {
-    if (aligned) scan_kernel<T, true, true><<<grid, block, 0, stream>>>(in, out, n, init, hdr, desc);
-    else         scan_kernel<T, true, false><<<grid, block, 0, stream>>>(in, out, n, init, hdr, desc);
-  } else {
-    if (aligned) scan_kernel<T, false, true><<<grid, block, 0, stream>>>(in, out, n, init, hdr, desc);
-    else         scan_kernel<T, false, false><<<grid, block, 0, stream>>>(in, out, n, init, hdr, desc);
-  }
+  if (exclusive) scan_kernel<T, true><<<grid, block, 0, stream>>>(in, out, n, init, hdr, desc);
+  else           scan_kernel<T, false><<<grid, block, 0, stream>>>(in, out, n, init, hdr, desc);
   trace_mark(stream, kTraceScan);
   return (int)cudaGetLastError();
 }
@@ -889,8 +859,8 @@ extern "C" int tb200_scan_static(const void* d_in, void* d_out, uint64_t n, int 
   rc = static_scan_scratch(&scratch);
   if (rc) return rc;
   size_t have = kStaticScanBytes;
-  // tb200_scan clears the part of the scratch it uses (header and descriptors) on `stream`
-  // before the kernel, so what the previous call left behind is never read.
+  // tb200_scan clears the part of the scratch that its kernel reads on `stream` (header and descriptors; a scan by one
+  // cluster reads none and sets the status word itself), so what the previous call left behind is never read.
   return tb200_scan(scratch, &have, d_in, d_out, n, dtype, exclusive, h_init, stream);
 }
 
