@@ -5,6 +5,7 @@ The inputs reach every decision: buckets that fit after one pass and after two, 
 keys outside the sampled window, a bucket above the capacity, 64-bit keys whose windows are equal, crowded bins.
 """
 import ctypes as C
+import threading
 
 import numpy as np
 import pytest
@@ -139,3 +140,67 @@ def test_keys_with_copies_are_not_slower_than_byte_wise(cuda_device, dtype):
     for copies in (4, 16, 40, 100):
         k0 = _copies(n, copies, dtype, cuda_device)
         assert device_time(k0, need.value) < 1.15 * device_time(k0, need.value - (1 << 19)), copies
+
+
+@pytest.mark.parametrize("dtype", [np.int32, np.float32, np.uint64])
+def test_descending_in_two_passes(cuda_device, dtype):
+    n = 4200001
+    k = random_keys(np.random.default_rng(8200), n, dtype)
+    v = np.arange(n, dtype=np.uint32)
+    dk, dv = to_device(k), to_device(v)
+    tb.sort_by_key(dk, dv, descending=True)
+    wk, wv = oracle.port().sort_by_key(k, v, True)
+    assert to_host(dk, dtype).tobytes() == wk.tobytes()
+    assert to_host(dv, np.uint32).tobytes() == wv.tobytes()
+
+
+# What the device decided, as the control block at the start of the scratch holds it: executed passes (word 2), whether
+# there is a plan (word 28), window bits (34), tiles (37) and the bits in which the keys of a tile differ (38).
+@pytest.mark.parametrize("kind,n,passes,tiles", [
+    ("uniform", 100003, 1, None), ("uniform", 4200001, 2, "even"), ("uniform", 3200001, 2, "cut"),
+    ("outlier", 4200001, None, None), ("heavy", 4200001, None, None)])
+def test_plans_that_the_device_chooses(cuda_device, kind, n, passes, tiles):
+    k = _keys(np.random.default_rng(8300), kind, n, np.uint64)
+    d = to_device(k)
+    need = C.c_size_t(0)
+    stream = C.c_void_p(torch.cuda.current_stream(cuda_device).cuda_stream)
+    args = (n, capi.U64, 0, 0, 0, 64, stream)
+    capi.check(capi.lib.tb200_radix_sort(None, C.byref(need), None, None, *args), "size")
+    temp = torch.empty(need.value, dtype=torch.uint8, device=cuda_device)
+    capi.check(capi.lib.tb200_radix_sort(C.c_void_p(temp.data_ptr()), C.byref(need), C.c_void_p(d.data_ptr()), None, *args),
+               "sort")
+    assert to_host(d, np.uint64).tobytes() == np.sort(k).tobytes()
+    word = to_host(temp[:160], np.uint32)
+    assert bool(word[28]) == (passes is not None)
+    if passes is not None:
+        assert word[2] == passes
+    if tiles == "even":  # groups of 2^g whole buckets
+        assert word[38] < word[34] and word[37] & (word[37] - 1) == 0
+    elif tiles == "cut":
+        assert word[38] == word[34] and word[37] & (word[37] - 1) != 0
+
+
+def test_sorts_of_several_threads_and_streams_at_once(cuda_device):
+    """The kernels of a sort are chained with dependent launches: those of other streams run in between."""
+    wrong = []
+
+    def work(i):
+        stream = torch.cuda.Stream(cuda_device)
+        with torch.cuda.stream(stream):
+            g = torch.Generator(device=cuda_device)
+            g.manual_seed(i)
+            for n in (700_001 + i, 5_000_011, 3000 + i):
+                k0 = torch.randint(-2**63, 2**63 - 1, (n,), dtype=torch.int64, device=cuda_device, generator=g)
+                want, order = torch.sort(k0, stable=True)
+                for _ in range(4):
+                    k, v = k0.clone(), torch.arange(n, dtype=torch.int32, device=cuda_device)
+                    tb.sort_by_key(k, v)
+                    if not (torch.equal(k, want) and torch.equal(v, order.to(torch.int32))):
+                        wrong.append((i, n))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
