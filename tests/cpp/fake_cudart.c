@@ -36,7 +36,3 @@ int cudaFreeHost(void* p) {
   free(p);
   return 0;
 }
-int cudaThreadExchangeStreamCaptureMode(int* mode) {
-  (void)mode;
-  return 0;
-}

@@ -120,13 +120,9 @@ unsigned char* landing_take() {
   std::lock_guard<std::mutex> lock(g_landing_mutex);
   if (!g_landing_asked) {
     g_landing_asked = true;
-    // another thread may be capturing a graph: the allocation has nothing to do with it and must not end it
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    cudaThreadExchangeStreamCaptureMode(&mode);
     void* p = nullptr;
     if (cudaHostAlloc(&p, kSlots * kSlotBytes, cudaHostAllocPortable) == cudaSuccess) g_landing_page = static_cast<unsigned char*>(p);
     else (void)cudaGetLastError();
-    cudaThreadExchangeStreamCaptureMode(&mode);
   }
   if (g_landing_page == nullptr || ~g_landing_taken == 0) return nullptr;
   const int slot = __builtin_ctzll(~g_landing_taken);
