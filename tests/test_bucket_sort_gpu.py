@@ -204,3 +204,18 @@ def test_sorts_of_several_threads_and_streams_at_once(cuda_device):
     for t in threads:
         t.join()
     assert not wrong
+
+
+@pytest.mark.parametrize("n,planned", [(237 * 4608, True), (237 * 4608 + 1, False), ((1 << 22) - 1, False), (1 << 22, True)])
+def test_plan_is_enqueued_where_there_can_be_one(cuda_device, n, planned):
+    """32-bit keys above what one pass can leave and below 2^22: the host knows that there is no plan."""
+    k = to_device(random_keys(np.random.default_rng(8400), n, np.uint32))
+    want = np.sort(to_host(k, np.uint32))
+    stream = C.c_void_p(torch.cuda.current_stream(cuda_device).cuda_stream)
+    ms, kinds = (C.c_float * 32)(), (C.c_int * 32)()
+    capi.check(capi.lib.tb200_trace_begin(stream), "trace")
+    tb.sort(k, key_dtype=capi.U32)
+    launches = capi.lib.tb200_trace_end(ms, kinds, 32)
+    assert 0 < launches <= 32
+    assert (14 in kinds[:launches]) == planned  # the plan's kernels
+    assert to_host(k, np.uint32).tobytes() == want.tobytes()

@@ -113,22 +113,3 @@ def test_nccl_library_exports_its_entry_point_and_answers_the_size_query():
     need = C.c_size_t(0)
     assert nccl_sort.lib.tb200_sample_sort(None, 3, 2, None, C.byref(need), None, None, 10, None, None, 10, None, None,
                                            None, None) == capi.ERR_INVALID_ARGUMENT  # rank outside the communicator
-
-
-def test_sorts_that_never_take_the_bucket_plan_ask_for_no_scratch_of_it():
-    """32-bit keys between one pass (237 tiles of 4608 keys) and 2^22 keys; the plan's counts and tiles take 512 KiB."""
-    from thrust_b200 import _capi as capi
-
-    def beside_the_arrays(n, dtype):
-        need = C.c_size_t(0)
-        assert capi.lib.tb200_radix_sort(None, C.byref(need), None, None, n, dtype, 4, 0, 0, 8 * capi.DTYPE_BYTES[dtype],
-                                         None) == 0
-        tile = 256 * (32 if capi.DTYPE_BYTES[dtype] == 4 else 24)
-        return need.value - n * (capi.DTYPE_BYTES[dtype] + 4) - -(-n // tile) * 1024
-
-    plan = 1 << 19
-    for n in (237 * 4608 + 1, 2_000_003, (1 << 22) - 1):
-        assert beside_the_arrays(n, capi.I32) < plan, n
-        assert beside_the_arrays(n, capi.I64) > plan, n
-    for n in (9217, 237 * 4608, 1 << 22, 1 << 25):
-        assert beside_the_arrays(n, capi.F32) > plan, n

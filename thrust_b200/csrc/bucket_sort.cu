@@ -191,7 +191,7 @@ bucket_prepare_kernel(const UK* __restrict__ keys, uint64_t n, Encoding enc, Sor
       while (bucket_bits < max_bits && (cell >> (bucket_bits - 12)) > capacity / 2) ++bucket_bits;
       ok = ok && (cell >> (bucket_bits - 12)) <= 2ull * capacity;
     }
-    // below kTwoPassMin 32-bit keys only a plan of one pass is worth its count (bucket_scratch_bytes)
+    // below kTwoPassMin 32-bit keys only a plan of one pass is worth its count (bucket_plan_possible)
     if (sizeof(UK) == 4 && n < kTwoPassMin) ok = ok && s_most <= 16;
     ctl->window_ok = ok;
     ctl->bucket_bits = (unsigned)bucket_bits;
@@ -568,13 +568,15 @@ int finish_vals(int vb, const SortCtl* ctl, const BucketScratch* scratch, void* 
 }  // namespace
 
 size_t bucket_scratch_bytes(uint64_t n, int key_bytes, int val_bytes) {
-  const int size = tile_size_of(n, val_bytes);
-  if (key_bytes < 4 || n < kSamples || size < 0) return 0;
-  // 32-bit keys have four byte-wise passes at most: below kTwoPassMin keys only a plan of one pass is worth its count, and
-  // one pass leaves 256 buckets: more than 237 times a tile's capacity cannot be expected to fit them all (evenly spread
-  // keys: a mean of 237 / 256 of the capacity leaves five standard deviations at 4608).
-  if (key_bytes == 4 && n < kTwoPassMin && n > 237 * capacity_of(size)) return 0;
+  if (key_bytes < 4 || n < kSamples || tile_size_of(n, val_bytes) < 0) return 0;
   return align_up(sizeof(BucketScratch), 256);
+}
+
+// 32-bit keys have four byte-wise passes at most: below kTwoPassMin keys only a plan of one pass is worth its count, and one
+// pass leaves 256 buckets: more than 237 times a tile's capacity cannot be expected to fit them all (evenly spread keys: a
+// mean of 237 / 256 of the capacity leaves five standard deviations at 4608).
+bool bucket_plan_possible(uint64_t n, int key_bytes, int val_bytes) {
+  return key_bytes != 4 || n >= kTwoPassMin || n <= 237 * capacity_of(tile_size_of(n, val_bytes));
 }
 
 int bucket_plan(void* d_ctl, size_t clear_bytes, void* d_bucket_scratch, const void* d_keys, uint64_t n, int key_bytes,

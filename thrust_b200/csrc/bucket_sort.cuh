@@ -17,6 +17,9 @@ template <> struct TileShape<2> { static constexpr int kThreads = 1024, kItems =
 // Scratch behind the radix sort's own for n elements (0: this size and these types take no bucket plan).
 size_t bucket_scratch_bytes(uint64_t n, int key_bytes, int val_bytes);
 
+// False: no keys of this size and type take a plan, and none need be enqueued (where there is scratch for one).
+bool bucket_plan_possible(uint64_t n, int key_bytes, int val_bytes);
+
 // First half, instead of clearing the scratch: clears [d_temp, d_temp + clear_bytes) (control block first), samples
 // the keys, counts the buckets and, when they fit, writes the plan into the control block.
 int bucket_plan(void* d_ctl, size_t clear_bytes, void* d_bucket_scratch, const void* d_keys, uint64_t n, int key_bytes,

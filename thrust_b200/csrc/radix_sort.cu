@@ -873,7 +873,8 @@ int sort_impl(void* d_temp, size_t* temp_bytes, void* d_keys, void* d_vals, uint
     return block_sort_single(d_keys, d_vals, n, sizeof(UK), VB, kind, descending, &ctl->status, stream);
   }
   // Larger whole-key sorts try a bucket plan first (a scratch sized for the byte-wise sort alone still serves that).
-  const bool buckets = phase == kPhaseAll && whole && bucket_bytes != 0 && *temp_bytes >= lay.total + bucket_bytes;
+  const bool buckets = phase == kPhaseAll && whole && bucket_bytes != 0 && *temp_bytes >= lay.total + bucket_bytes &&
+                       bucket_plan_possible(n, sizeof(UK), VB);
   if (buckets) {
     if (d_keys == nullptr || (VB && d_vals == nullptr)) return TB200_ERR_INVALID_ARGUMENT;
     const int rc = bucket_plan(ctl, lay.clear_bytes, base + lay.total, d_keys, n, sizeof(UK), VB, kind, descending, stream);
