@@ -6,8 +6,8 @@
 namespace tb200 {
 
 // Threads, items per thread, bins and CTAs per SM of the tile sort, smallest capacity first. The tile sort is bound by
-// shared-memory wavefronts and issue slots together (about 9 us per tile of 4096 pairs and CTA, 2 CTAs per SM, 2^28
-// (u64,u32) pairs: 2.0 ms at 3.2 TB/s); 8192 bins (0.4 % slower), 768 x 6 (3 % slower), 512 x 9 three times per SM with
+// shared-memory wavefronts (77 % of that pipe's peak; issue slots 40 %, DRAM 44 %: 2^26 (u64,u32) pairs; about 9 us per
+// tile of 4096 pairs and CTA, 2 CTAs per SM, 2^28 pairs: 2.0 ms at 3.2 TB/s; shape 2 takes 12.5 ms for 2^30); 8192 bins (0.4 % slower), 768 x 6 (3 % slower), 512 x 9 three times per SM with
 // 40 registers (5 % slower on 64-bit keys) and 384 x 12 (equal) were tried.
 template <int SIZE> struct TileShape;
 template <> struct TileShape<0> { static constexpr int kThreads = 512, kItems = 9, kBins = 16384, kMinCtas = 2; };
