@@ -91,24 +91,16 @@ __device__ void look_for_copies(const UK* __restrict__ keys, uint64_t n, int ali
 #pragma unroll
   for (int p = 0; p < kParts; ++p) {
     if (p >= (int)parts) break;
-    unsigned look = 0, hash[kMine], old[kMine];
 #pragma unroll
     for (int i = 0; i < kMine; ++i) {
-      hash[i] = (unsigned)key[p][i] * 2654435761u;
-      if (i % VEC != 0 && key[p][i] == key[p][i % VEC != 0 ? i - 1 : i]) ++beside;
-      else if ((hash[i] >> 17 & (parts - 1)) == 0) look |= 1u << i;
-    }
-#pragma unroll
-    for (int probe = 0; probe < 2; ++probe) {  // the keys of a thread side by side
-#pragma unroll
-      for (int i = 0; i < kMine; ++i)
-        if (look >> i & 1u) old[i] = atomicCAS(&s_seen[((hash[i] >> 19) + probe) % kSamples], 0u, (unsigned)key[p][i]);
-#pragma unroll
-      for (int i = 0; i < kMine; ++i) {
-        if ((look >> i & 1u) && (old[i] == 0 || old[i] == (unsigned)key[p][i])) {
-          again += old[i] != 0;
-          look &= ~(1u << i);
-        }
+      const unsigned k = (unsigned)key[p][i], hash = k * 2654435761u;
+      if (i % VEC != 0 && key[p][i] == key[p][i % VEC != 0 ? i - 1 : i]) { ++beside; continue; }
+      if ((hash >> 17 & (parts - 1)) != 0) continue;
+      for (unsigned probe = 0; probe < 2; ++probe) {
+        unsigned* cell = &s_seen[((hash >> 19) + probe) % kSamples];
+        unsigned old = *(volatile unsigned*)cell;  // a frequent key is there as a rule: no queue of atomics on its cell
+        if (old == 0) old = atomicCAS(cell, 0u, k);
+        if (old == 0 || old == k) { again += old != 0; break; }
       }
     }
   }
